@@ -18,7 +18,7 @@ import torch.nn as nn
 
 from ..ops import gemm as G
 from ..ops.attention import flash_attention, flash_attention_packed
-from ..ops.cross_entropy import softmax_cross_entropy
+from ..ops.cross_entropy import next_token_cross_entropy
 from ..ops.elementwise import dropout, embedding_sum
 from ..ops.linear import linear as k_linear, mlp as k_mlp
 from ..ops.modules import Dropout, Embedding, LayerNorm, Linear
@@ -181,7 +181,7 @@ class GPT2LMHeadModel(nn.Module):
         logits = self.lm_head(h)
         if labels is None:
             return logits
-        loss = softmax_cross_entropy(logits[:, :-1, :], labels[:, 1:])
+        loss = next_token_cross_entropy(logits, labels)
         return loss, logits
 
 

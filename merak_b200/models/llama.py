@@ -17,7 +17,7 @@ import torch
 import torch.nn as nn
 
 from ..ops.attention import flash_attention
-from ..ops.cross_entropy import softmax_cross_entropy
+from ..ops.cross_entropy import next_token_cross_entropy
 from ..ops.elementwise import apply_rope, rope_tables, swiglu
 from ..ops.modules import Embedding, Linear, RMSNorm, expose_fused_projection
 
@@ -149,7 +149,7 @@ class LlamaForCausalLM(nn.Module):
         logits = self.lm_head(h)
         if labels is None:
             return logits
-        return softmax_cross_entropy(logits[:, :-1, :], labels[:, 1:]), logits
+        return next_token_cross_entropy(logits, labels), logits
 
 
 def llama_config(name: str = "llama-7b", **overrides) -> LlamaConfig:

@@ -19,7 +19,7 @@ import torch.nn as nn
 import torch.nn.functional as F
 
 from ..ops.attention import flash_attention
-from ..ops.cross_entropy import softmax_cross_entropy
+from ..ops.cross_entropy import next_token_cross_entropy
 from ..ops.elementwise import apply_rope, rope_tables, swiglu
 from ..ops.modules import Embedding, Linear, RMSNorm, expose_fused_projection
 from ..parallel.expert import MoELayer
@@ -202,7 +202,7 @@ class DeepseekV2ForCausalLM(nn.Module):
         logits = self.lm_head(h)
         if labels is None:
             return logits
-        loss = softmax_cross_entropy(logits[:, :-1, :], labels[:, 1:])
+        loss = next_token_cross_entropy(logits, labels)
         aux = self.aux_loss()
         if aux is not None:
             loss = loss + aux.to(loss.dtype)

@@ -86,3 +86,18 @@ def softmax_cross_entropy(logits: torch.Tensor, labels: torch.Tensor, ignore_ind
                                                          ignore_index) * loss_scale
         return cross_entropy_reference(logits, labels, ignore_index) * loss_scale
     return _SoftmaxCrossEntropy.apply(logits, labels, ignore_index, vocab_start, tp_group, loss_scale)
+
+
+def next_token_cross_entropy(logits: torch.Tensor, labels: torch.Tensor, ignore_index: int = -100,
+                             vocab_start: int = 0, tp_group=None) -> torch.Tensor:
+    """Mean cross entropy of ``logits[:, t]`` against ``labels[:, t + 1]``.
+
+    The labels move instead of the logits: the kernels see every row where the GEMM wrote it, with "no target" at
+    the last position.  Slicing the logits costs a copy of them in the forward pass (two when the vocabulary is
+    not a multiple of 8) and a zero-filled tensor, a copy and the re-pitching copies of two GEMMs in the backward
+    pass; at 8 x 1024 x 50257 that was 5.2 ms per micro-batch."""
+    if (not _lib.use_kernels(logits) or logits.dtype not in (torch.bfloat16, torch.float32) or logits.dim() != 3
+            or labels.shape != logits.shape[:2] or logits.shape[1] < 2):
+        return softmax_cross_entropy(logits[:, :-1, :], labels[:, 1:], ignore_index, vocab_start, tp_group)
+    shifted = F.pad(labels[:, 1:], (0, 1), value=ignore_index)
+    return softmax_cross_entropy(logits, shifted, ignore_index, vocab_start, tp_group)

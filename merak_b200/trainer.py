@@ -22,7 +22,7 @@ from torch.utils.data import DataLoader, Dataset
 
 from . import initialize
 from .args import MerakArguments, manual_set_args, mergeargs, print_args
-from .ops.cross_entropy import softmax_cross_entropy
+from .ops.cross_entropy import next_token_cross_entropy, softmax_cross_entropy
 from .parallel import mpu
 from .pipeline.engine import PipelineEngine
 from .pipeline.module import PipelineModule
@@ -142,15 +142,11 @@ class MerakTrainer:
                 logits = logits["logits"] if "logits" in logits else next(iter(logits.values()))
             if isinstance(labels, dict):
                 labels = labels.get("labels", next(iter(labels.values())))
-            if causal:
-                logits, labels = logits[:, :-1, :], labels[:, 1:]
+            cross_entropy = next_token_cross_entropy if causal else softmax_cross_entropy
             if parallel_vocab:
                 start = mpu.get_model_parallel_rank() * logits.shape[-1]
-                return softmax_cross_entropy(logits, labels, vocab_start=start,
-                                             tp_group=mpu.get_model_parallel_group())
-            if logits.dim() == 2 and labels.dim() == 1:
-                return softmax_cross_entropy(logits, labels)
-            return softmax_cross_entropy(logits, labels)
+                return cross_entropy(logits, labels, vocab_start=start, tp_group=mpu.get_model_parallel_group())
+            return cross_entropy(logits, labels)
         return loss_fn
 
     def _is_causal(self) -> bool:
