@@ -16,9 +16,9 @@ from typing import Optional
 import torch
 import torch.nn as nn
 
-from ..ops.attention import flash_attention
+from ..ops.attention import rope_attention_packed
 from ..ops.cross_entropy import next_token_cross_entropy
-from ..ops.elementwise import apply_rope, rope_tables, swiglu
+from ..ops.elementwise import rope_tables, swiglu
 from ..ops.modules import Embedding, Linear, RMSNorm, expose_fused_projection
 
 
@@ -70,10 +70,9 @@ class LlamaAttention(nn.Module):
         kv_local = qkv.shape[-1] // ((ratio + 2) * self.head_dim)      # local kv heads under TP
         q_local = kv_local * ratio
         qkv = qkv.view(B, L, q_local + 2 * kv_local, self.head_dim)
-        q, k, v = qkv[:, :, :q_local], qkv[:, :, q_local:q_local + kv_local], qkv[:, :, q_local + kv_local:]
         cos, sin = self._tables(x.device)
-        q, k = apply_rope(q, cos, sin, position_ids), apply_rope(k, cos, sin, position_ids)
-        ctx = flash_attention(q, k, v, causal=True).reshape(B, L, q_local * self.head_dim)
+        ctx = rope_attention_packed(qkv, q_local, kv_local, cos, sin, position_ids)
+        ctx = ctx.reshape(B, L, q_local * self.head_dim)
         return self.o_proj(ctx, residual) if type(self.o_proj) is Linear else (
             self.o_proj(ctx) if residual is None else self.o_proj(ctx) + residual)
 

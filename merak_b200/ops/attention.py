@@ -19,6 +19,7 @@ import torch
 import torch.nn.functional as F
 
 from . import _lib, flop_counter
+from .elementwise import _rope_launch, apply_rope
 from .rng import dropout_state
 
 def _declare():
@@ -204,6 +205,71 @@ class _FlashAttentionPacked(torch.autograd.Function):
             call_id, _lib.stream_ptr())
         _lib.check(rc, "mrk_attn_bwd")
         return dqkv, None, None, None, None, None, None
+
+
+class _RopeAttentionPacked(torch.autograd.Function):
+    """Rotary embedding of the query and key heads, then attention, on one packed projection output.  Forward: one
+    rotation launch writes the rotated heads, the value heads are read where the GEMM wrote them.  Backward: the
+    attention writes dQ, dK and dV into one packed gradient and one launch rotates its query and key heads back in
+    place, so the projection gets its gradient without slices of it being zero-filled, copied and summed."""
+
+    @staticmethod
+    def forward(ctx, qkv, hq, hkv, cos, sin, positions, causal, scale):
+        if not _tma_ok(qkv):
+            qkv = qkv.contiguous()
+        B, L, _, D = qkv.shape
+        qk = _rope_launch(qkv[:, :, :hq + hkv], cos, sin, positions, False)
+        q, k, v = qk[:, :, :hq], qk[:, :, hq:], qkv[:, :, hq + hkv:]
+        out = torch.empty((B, L, hq, D), dtype=qkv.dtype, device=qkv.device)
+        lse = torch.empty((B, hq, L), dtype=torch.float32, device=qkv.device)
+        rc = _lib.kernels().mrk_attn_fwd(
+            q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr(), lse.data_ptr(), 0, B, hq, hkv, L, L, D,
+            *_strides3(q), *_strides3(k), *_strides3(v), *_strides3(out), int(causal), float(scale), _lib.stream_ptr())
+        _lib.check(rc, "mrk_attn_fwd")
+        ctx.save_for_backward(qk, qkv, out, lse, cos, sin, positions)
+        ctx.meta = (hq, hkv, causal, scale)
+        return out
+
+    @staticmethod
+    def backward(ctx, dout):
+        qk, qkv, out, lse, cos, sin, positions = ctx.saved_tensors
+        hq, hkv, causal, scale = ctx.meta
+        B, L, _, D = qkv.shape
+        if not _tma_ok(dout):
+            dout = dout.contiguous()
+        q, k, v = qk[:, :, :hq], qk[:, :, hq:], qkv[:, :, hq + hkv:]
+        dqkv = torch.empty((B, L, hq + 2 * hkv, D), dtype=qkv.dtype, device=qkv.device)
+        dq, dk, dv = dqkv[:, :, :hq], dqkv[:, :, hq:hq + hkv], dqkv[:, :, hq + hkv:]
+        delta = torch.empty((B, hq, L), dtype=torch.float32, device=qkv.device)
+        dq_acc = torch.empty((B, L, hq, D), dtype=torch.float32, device=qkv.device)
+        strides = []
+        for t in (q, k, v, out, dout, dq, dk, dv):
+            strides.extend(_strides3(t))
+        arr = (ctypes.c_longlong * 24)(*strides)
+        rc = _lib.kernels().mrk_attn_bwd(
+            q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr(), dout.data_ptr(), lse.data_ptr(),
+            delta.data_ptr(), dq_acc.data_ptr(), dq.data_ptr(), dk.data_ptr(), dv.data_ptr(), 0,
+            B, hq, hkv, L, L, D, ctypes.cast(arr, ctypes.c_void_p), int(causal), float(scale), _lib.stream_ptr())
+        _lib.check(rc, "mrk_attn_bwd")
+        dqk = dqkv[:, :, :hq + hkv]
+        _rope_launch(dqk, cos, sin, positions, True, out=dqk)
+        return dqkv, None, None, None, None, None, None, None
+
+
+def rope_attention_packed(qkv: torch.Tensor, num_q_heads: int, num_kv_heads: int, cos: torch.Tensor,
+                          sin: torch.Tensor, positions: Optional[torch.Tensor] = None,
+                          causal: bool = True) -> torch.Tensor:
+    """Self-attention on ``qkv`` of shape ``[B, L, Hq + 2*Hkv, D]`` after rotary embedding of its query and key
+    heads (:func:`~merak_b200.ops.elementwise.apply_rope`); returns ``[B, L, Hq, D]``."""
+    D = qkv.shape[-1]
+    if not _lib.use_kernels(qkv) or qkv.dtype != torch.bfloat16 or D not in (64, 128):
+        q, k, v = (qkv[:, :, :num_q_heads], qkv[:, :, num_q_heads:num_q_heads + num_kv_heads],
+                   qkv[:, :, num_q_heads + num_kv_heads:])
+        q, k = apply_rope(q, cos, sin, positions), apply_rope(k, cos, sin, positions)
+        return flash_attention(q, k, v, causal=causal)
+    if flop_counter.enabled():
+        flop_counter.add(4 * qkv.shape[0] * num_q_heads * qkv.shape[1] * qkv.shape[1] * D // (2 if causal else 1))
+    return _RopeAttentionPacked.apply(qkv, num_q_heads, num_kv_heads, cos, sin, positions, causal, 1.0 / math.sqrt(D))
 
 
 def flash_attention_packed(qkv: torch.Tensor, num_q_heads: int, num_kv_heads: int,

@@ -159,11 +159,11 @@ def rope_reference(x, cos, sin, positions=None, inverse=False):
     return torch.cat([lo * c - hi * s, hi * c + lo * s], dim=-1).to(x.dtype)
 
 
-def _rope_launch(x, cos, sin, positions, inverse):
+def _rope_launch(x, cos, sin, positions, inverse, out=None):
     B, L, H, D = x.shape
     if x.stride(3) != 1:
         x = x.contiguous()
-    y = torch.empty((B, L, H, D), dtype=x.dtype, device=x.device)
+    y = out if out is not None else torch.empty((B, L, H, D), dtype=x.dtype, device=x.device)    # may be x itself
     pos = positions.to(torch.int64).contiguous() if positions is not None else None
     _lib.check(_lib.kernels().mrk_rope(x.data_ptr(), y.data_ptr(), cos.data_ptr(), sin.data_ptr(), _lib.ptr(pos),
                                        B, L, H, D, x.stride(0), x.stride(1), x.stride(2), y.stride(0), y.stride(1),
