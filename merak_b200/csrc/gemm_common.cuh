@@ -73,6 +73,7 @@ struct GemmParams {
   float alpha;
   unsigned* status;
   int num_m_blocks, num_n_blocks, num_k_blocks;
+  int full_tiles, num_units;      // pair kernel: tiles that run 256 columns wide; all units of one K range
   int num_splits, kb_per_split;   // split-K: work unit = (tile, split); partial sums meet in fp32 red.add
   int tma_store;                  // C leaves through shared memory + the TMA unit: 1 = bf16 stores (no accumulate), 2 = fp32 stores or adds
   int tma_store_aux;              // ... and the pre-activation side output too (second tensor map)

@@ -286,7 +286,7 @@ static int gemm_entry(const void* A, const void* B, void* C, int M, int N, int K
     if (N <= 64) bn = 64;
   }
   MRK_REQUIRE(bn == 64 || bn == 128 || bn == 256 || bn == 512, "gemm: block_n must be 64, 128, 256 or 512");
-  const int b_box_rows = bn == 512 ? 128 : bn;
+  const int b_box_rows = bn == 512 ? 64 : bn;
   CUtensorMap ta, tb;
   int rc;
   if (!a_mn) rc = make_tmap_2d(&ta, A, 2, (uint64_t)K, (uint64_t)M, (uint64_t)lda, kBlockK, kBlockM, 3);

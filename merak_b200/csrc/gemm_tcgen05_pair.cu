@@ -28,8 +28,15 @@ constexpr int kPairThreads = 320;     // TMA warp, UMMA warp, 8 epilogue warps
 // commit, the worse), one per eight 128.
 constexpr int kPairGroup = 2;
 constexpr int kPairStages = 3;
+// Time of a 256-column and of a 128-column unit, relative: half the products, but A is loaded in full (24 instead of
+// 32 KB per k-block for half the math) and the fill and the drain of a unit stay.  Measured on B200, whole tiles
+// only -> with halves where the rule takes them: 8192x3072x768 87 -> 75 us, 16384x1024x1024 45 -> 42, 8192x50257x768
+// 605 -> 560, 3003x2048x2048 48 -> 44; at a cost of 50 the rule also halves tiles of long products that lose by it
+// (4096x4096x11008 259 -> 286 us), at 75 it leaves 8192x3072x768 whole.
+constexpr int kPairFullCost = 100, kPairHalfCost = 60;
 constexpr int kPairABytes = 128 * kPairBlockK * 2;            // this CTA's rows of A, one k-block
 constexpr int kPairBBytes = (kPairBlockN / 2) * kPairBlockK * 2;  // this CTA's half of B, one k-block
+constexpr int kPairBBoxBytes = 64 * kPairBlockK * 2;          // one 64-column box of it, in either operand layout
 constexpr int kPairSubBytes = kPairABytes + kPairBBytes;      // 32 KB per k-block
 constexpr int kPairStageBytes = kPairGroup * kPairSubBytes;   // 64 KB
 // epilogue staging: one 128-row x 64-column bf16 box (TMA-store source) per column half
@@ -254,6 +261,31 @@ __device__ __forceinline__ void rs_reducer_role(const GemmParams& p, uint8_t* sm
     rs_pull_consumer(p, smem, ring_bytes, pull_full, pull_empty, slot_piece, abort_flag);
 }
 
+// Unit -> rows and columns.  The first `full_tiles` units are 256-column tiles in raster order; every tile after
+// those is two units of 128 columns, and the last num_m_blocks units (when N ends at most 128 columns into a
+// tile) are the 128-column units of that last strip.
+__device__ __forceinline__ void pair_unit(const GemmParams& p, int u, int& m_blk, int& col0, int& cols) {
+  const int tiles = p.num_m_blocks * p.num_n_blocks;
+  const int halves = 2 * (tiles - p.full_tiles);
+  cols = kPairBlockN;
+  int tile = u, shift = 0;
+  if (u >= p.full_tiles) {
+    const int h = u - p.full_tiles;
+    cols = kPairBlockN / 2;
+    tile = p.full_tiles + (h >> 1);
+    shift = (h & 1) * (kPairBlockN / 2);
+    if (h >= halves) {
+      m_blk = h - halves;
+      col0 = p.num_n_blocks * kPairBlockN;
+      return;
+    }
+  }
+  int n_blk;
+  tile_coords(tile, p.num_m_blocks, p.num_n_blocks, m_blk, n_blk);
+  m_blk = comm_perm_m(p, m_blk, kPairBlockM);
+  col0 = n_blk * kPairBlockN + shift;
+}
+
 __global__ void __launch_bounds__(kPairThreads, 1)
 gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ CUtensorMap tma_b,
                       const __grid_constant__ CUtensorMap tma_c, const __grid_constant__ CUtensorMap tma_aux,
@@ -332,7 +364,7 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_co
   const int num_clusters = (p.comm.mode != 0 ? p.comm.gemm_ctas : (int)gridDim.x) >> 1;
   const bool rs = p.comm.mode == 1;
   // reduce-only launches (single-GPU tests of the reduce phase) skip the multiplication
-  const int num_units = (rs && p.comm.phase == 2) ? 0 : p.num_m_blocks * p.num_n_blocks * p.num_splits;
+  const int num_units = (rs && p.comm.phase == 2) ? 0 : p.num_units * p.num_splits;
 
   if (warp == 0) {
     // ------------------------------- TMA producer (both CTAs) -------------------------------
@@ -344,11 +376,11 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_co
       uint32_t phase = 0;
       bool ok = true;
       for (int unit = cluster_id; unit < num_units && ok; unit += num_clusters) {
-        int m_blk, n_blk;
-        tile_coords(unit / p.num_splits, p.num_m_blocks, p.num_n_blocks, m_blk, n_blk);
-        m_blk = comm_perm_m(p, m_blk, kPairBlockM);
+        int m_blk, col0, cols;
+        pair_unit(p, unit / p.num_splits, m_blk, col0, cols);
         const int m0 = m_blk * kPairBlockM + (int)cta * 128;
-        const int n0 = n_blk * kPairBlockN + (int)cta * (kPairBlockN / 2);
+        const int n0 = col0 + (int)cta * (cols / 2);
+        const int b_boxes = cols / 128;                 // 64-column boxes of B this CTA loads: 2 or 1
         const int kb_begin = (unit % p.num_splits) * p.kb_per_split;
         const int kb_end = min(p.num_k_blocks, kb_begin + p.kb_per_split);
         if (p.comm.mode == 2 && m0 < p.M) {       // this CTA's 128 rows of A must have arrived
@@ -360,7 +392,7 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_co
           ok = mbar_wait(smem_u32(&empty_bar[stage]), phase ^ 1u, abort_flag, p.status);
           if (!ok) break;
           const uint32_t fb = smem_u32(&full_bar[stage]);
-          if (leader) mbar_arrive_expect_tx(fb, (uint32_t)(nsub * 2 * kPairSubBytes));   // bytes of both CTAs
+          if (leader) mbar_arrive_expect_tx(fb, (uint32_t)(nsub * 2 * (kPairABytes + b_boxes * kPairBBoxBytes)));   // bytes of both CTAs
           for (int sub = 0; sub < nsub; ++sub) {
             const uint32_t sa = smem_u32(smem + stage * kPairStageBytes + sub * kPairSubBytes);
             const uint32_t sb = sa + kPairABytes;
@@ -372,13 +404,9 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_co
               for (int atom = 0; atom < 2; ++atom)
                 tma_load_2d_pair(sa + atom * (kPairBlockK * 128), &tma_a, fb, m0 + atom * 64, k0);
             }
-            if (!b_mn) {
-              tma_load_2d_pair(sb, &tma_b, fb, k0, n0);
-            } else {
-#pragma unroll
-              for (int atom = 0; atom < 2; ++atom)
-                tma_load_2d_pair(sb + atom * (kPairBlockK * 128), &tma_b, fb, n0 + atom * 64, k0);
-            }
+            for (int box = 0; box < b_boxes; ++box)
+              tma_load_2d_pair(sb + box * kPairBBoxBytes, &tma_b, fb, b_mn ? n0 + box * 64 : k0,
+                               b_mn ? k0 : n0 + box * 64);
           }
           if (++stage == kPairStages) { stage = 0; phase ^= 1u; }
         }
@@ -397,7 +425,6 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_co
   } else if (warp == 1) {
     // ------------------------------- UMMA issuer (leader CTA) -------------------------------
     if (lane == 0 && leader) {
-      const uint32_t idesc = make_idesc_bf16(kPairBlockM, kPairBlockN, a_mn ? 1u : 0u, b_mn ? 1u : 0u);
       int stage = 0;
       uint32_t phase = 0;
       int iter = 0;
@@ -405,6 +432,9 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_co
       for (int unit = cluster_id; unit < num_units && ok; unit += num_clusters, ++iter) {
         const int acc = iter & 1;
         const uint32_t acc_phase = (iter >> 1) & 1;
+        int m_blk, col0, cols;
+        pair_unit(p, unit / p.num_splits, m_blk, col0, cols);
+        const uint32_t idesc = make_idesc_bf16(kPairBlockM, (uint32_t)cols, a_mn ? 1u : 0u, b_mn ? 1u : 0u);
         ok = mbar_wait(smem_u32(&tmem_empty_bar[acc]), acc_phase ^ 1u, abort_flag, p.status);
         if (!ok) break;
         tc_fence_after();
@@ -466,9 +496,8 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_co
       box_busy = true;
     };
     for (int unit = cluster_id; unit < num_units && ok; unit += num_clusters, ++iter) {
-      int m_blk, n_blk;
-      tile_coords(unit / p.num_splits, p.num_m_blocks, p.num_n_blocks, m_blk, n_blk);
-      m_blk = comm_perm_m(p, m_blk, kPairBlockM);
+      int m_blk, col0, cols;
+      pair_unit(p, unit / p.num_splits, m_blk, col0, cols);
       const bool split_k = p.num_splits > 1;
       const bool first_split = (unit % p.num_splits) == 0;
       const int acc = iter & 1;
@@ -477,11 +506,12 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_co
       const long long row = row0 + row_in_tile;
       const bool row_ok = row < p.M;
       const uint32_t t_row = tmem_base + ((uint32_t)(quad * 32) << 16) + acc * kPairBlockN;
-      const int col_half = n_blk * kPairBlockN + half * (kPairBlockN / 2);
+      const int width = cols / 2;                    // columns of each epilogue half: 128 or 64
+      const int col_half = col0 + half * width;
       // staged output for this block? (uniform over the four warps of the half)
       const bool staged32 = p.tma_store == 2 && col_half < p.N;     // fp32 output: boxes of 32 columns
       const bool staged = p.tma_store == 1 && !split_k && col_half < p.N &&
-                          (col_half + kPairBlockN / 2 <= p.N || (p.aux_mode == MRK_AUX_NONE && p.aux_out == nullptr));
+                          (col_half + width <= p.N || (p.aux_mode == MRK_AUX_NONE && p.aux_out == nullptr));
       // aux_in (residual, or the saved pre-activation of a backward GEMM) comes into the box by TMA
       const bool aux_tma = staged && p.tma_aux_in && p.aux_mode != MRK_AUX_NONE &&
                            !(p.tma_store_aux && p.aux_out != nullptr);
@@ -512,10 +542,10 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_co
       };
       if (staged) {
         const bool two_pass = p.tma_store_aux && p.aux_out != nullptr;
-        const int npass = (col_half + 64 < p.N) ? 2 : 1;        // 64-column passes with anything to write
+        const int npass = (width == 128 && col_half + 64 < p.N) ? 2 : 1;        // 64-column passes with anything to write
         for (int b = 0; b < npass; ++b) {
           const int col_b = col_half + b * 64;
-          const uint32_t t_b = t_row + half * (kPairBlockN / 2) + b * 64;
+          const uint32_t t_b = t_row + half * width + b * 64;
           if (two_pass) {
             // the pre-activation side output of these columns first, through the same box
             box_acquire();
@@ -540,18 +570,18 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_co
           box_store(&tma_c, col_b, row0);
         }
         if (rs && store_thread && row0 < p.M) {
-          pending_flag = ((m_blk * p.num_n_blocks + n_blk) * 2 + (int)cta) * 2 + half;
+          pending_flag = ((m_blk * p.num_n_blocks + col0 / kPairBlockN) * 2 + (int)cta) * 2 + half;
           pending_owner = (int)((row0 / p.comm.seg_rows) % p.comm.n);
         }
       } else if (staged32) {
         // fp32 output through the same box, 32 columns (one 128-byte row per output row) at a time: a plain
         // store, or an element-wise add when the GEMM accumulates into its output or splits K
         const bool add = split_k || (p.flags & MRK_GEMM_ACCUMULATE) != 0;
-        const int npass = min(4, (p.N - col_half + 31) / 32);
+        const int npass = min(width / 32, (p.N - col_half + 31) / 32);
         for (int b = 0; b < npass; ++b) {
           const int col_b = col_half + b * 32;
           box_acquire();
-          epilogue_tile(p, row, row_ok, t_row + half * (kPairBlockN / 2) + b * 32, col_b, 32, split_k, first_split,
+          epilogue_tile(p, row, row_ok, t_row + half * width + b * 32, col_b, 32, split_k, first_split,
                         stage, row_in_tile, 3);
           if (b == npass - 1) release_tmem();
           fence_proxy_async_smem();
@@ -566,7 +596,7 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_co
           box_busy = true;
         }
       } else {
-        epilogue_tile(p, row, row_ok, t_row + half * (kPairBlockN / 2), col_half, kPairBlockN / 2, split_k,
+        epilogue_tile(p, row, row_ok, t_row + half * width, col_half, width, split_k,
                       first_split, nullptr, row_in_tile, 0);
         release_tmem();
       }
@@ -595,6 +625,27 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_co
   }
 }
 
+// How many of the tiles run whole: all of them, or as many as fill whole rounds of the clusters, the others
+// halved so that the last round spreads over twice as many clusters.
+static int pair_full_tiles(int tiles, int strip, int clusters) {
+  const int rounds = tiles / clusters;
+  const int options[4] = {tiles, rounds * clusters, rounds > 0 ? (rounds - 1) * clusters : 0, 0};
+  int best = tiles;
+  long long best_cost = 0;
+  for (int o = 0; o < 4; ++o) {
+    const int full = options[o], halves = 2 * (tiles - full) + strip;
+    long long cost = 0;                               // of the cluster with most to do; units go round robin
+    for (int c = 0; c < clusters; ++c) {
+      const long long nf = c < full ? (full - 1 - c) / clusters + 1 : 0;
+      const long long all = c < full + halves ? (full + halves - 1 - c) / clusters + 1 : 0;
+      const long long t = nf * kPairFullCost + (all - nf) * kPairHalfCost;
+      if (t > cost) cost = t;
+    }
+    if (o == 0 || cost < best_cost) { best_cost = cost; best = full; }
+  }
+  return best;
+}
+
 int launch_gemm_pair(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& tc, const CUtensorMap& taux,
                      const CUtensorMap& tauxin, GemmParams& p, cudaStream_t stream) {
   static bool configured[64] = {false};
@@ -608,8 +659,14 @@ int launch_gemm_pair(const CUtensorMap& ta, const CUtensorMap& tb, const CUtenso
   p.num_m_blocks = (p.M + kPairBlockM - 1) / kPairBlockM;
   p.num_n_blocks = (p.N + kPairBlockN - 1) / kPairBlockN;
   p.num_k_blocks = (p.K + kPairBlockK - 1) / kPairBlockK;
-  const int tiles = p.num_m_blocks * p.num_n_blocks;
   const int max_clusters = sm_count() / 2;
+  int strip = 0;          // 128-column units of a last strip that is at most half a tile wide
+  const int n_rem = p.N % kPairBlockN;
+  if (p.comm.mode == 0 && n_rem > 0 && n_rem <= kPairBlockN / 2 && p.N > kPairBlockN) {
+    --p.num_n_blocks;
+    strip = p.num_m_blocks;
+  }
+  const int tiles = p.num_m_blocks * p.num_n_blocks;
   p.num_splits = 1;
   const bool can_split = (p.flags & MRK_GEMM_OUT_F32) && (p.flags & MRK_GEMM_ACCUMULATE) &&
                          p.act == MRK_ACT_NONE && p.aux_mode == MRK_AUX_NONE && p.aux_out == nullptr;
@@ -622,14 +679,17 @@ int launch_gemm_pair(const CUtensorMap& ta, const CUtensorMap& tb, const CUtenso
     for (int sp = 1; sp <= 32 && sp <= max_by_k; ++sp) {
       const int kb = (p.num_k_blocks + sp - 1) / sp;
       const int nsp = (p.num_k_blocks + kb - 1) / kb;
-      const long long rounds = ((long long)tiles * nsp + max_clusters - 1) / max_clusters;
+      const long long rounds = ((long long)(2 * tiles + strip) * nsp + 2 * max_clusters - 1) / (2 * max_clusters);
       const long long cost = rounds * (kb + 6);
       if (sp == 1 || cost < best_cost) { best_cost = cost; p.num_splits = nsp; }
     }
   }
   p.kb_per_split = (p.num_k_blocks + p.num_splits - 1) / p.num_splits;
   p.num_splits = (p.num_k_blocks + p.kb_per_split - 1) / p.kb_per_split;
-  const int units = tiles * p.num_splits;
+  p.full_tiles = tiles;
+  if (p.comm.mode == 0 && p.num_splits == 1) p.full_tiles = pair_full_tiles(tiles, strip, max_clusters);
+  p.num_units = p.full_tiles + 2 * (tiles - p.full_tiles) + strip;
+  const int units = p.num_units * p.num_splits;
   int clusters = units < max_clusters ? units : max_clusters;
   int gather_clusters = 0;
   if (p.comm.mode == 2) {
