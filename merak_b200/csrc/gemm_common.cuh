@@ -225,15 +225,9 @@ __device__ __forceinline__ void tile_coords(int tile, int num_m, int num_n, int&
 // Epilogue of one accumulator tile for one thread: `row` is this thread's output row, `t_row` the
 // TMEM address of its lane at the tile's first column, `col_base` the first output column of the
 // tile and `ncols` its width.  All 32 lanes of the warp call this together.
-// `stage` (optional): shared-memory staging of this warp group's 128 x 128 output block, laid out as
-// two 128-row x 64-column boxes in the 128-byte TMA swizzle; when given, the finished bf16 values go
-// there (row `r_in_tile`) instead of to global memory and the caller issues the TMA stores.  The
-// caller only passes it for tiles where that is legal (bf16 output, no accumulate, no split-K, and
-// either a full-width block or no side tensors).
 template <int kAct, int kAux>
 __device__ __noinline__ void epilogue_tile_t(const GemmParams& p, long long row, bool row_ok, uint32_t t_row,
-                                              int col_base, int ncols, bool split_k, bool first_split,
-                                              uint8_t* stage, int r_in_tile, int pass) {
+                                              int col_base, int ncols, bool split_k, bool first_split) {
   const bool out_f32 = (p.flags & MRK_GEMM_OUT_F32) != 0;
   const bool accumulate = (p.flags & MRK_GEMM_ACCUMULATE) != 0;
   const bool bias_f32 = (p.flags & MRK_GEMM_BIAS_F32) != 0;
@@ -295,74 +289,6 @@ for (int h = 0; h < 2; ++h) {
           if (full || col0 + j < p.N) v[j] += __bfloat162float(__ldg(b + j));
       }
     }
-  }
-  if (stage != nullptr) {
-    // shared-memory staged output: side tensors are only present on full-width blocks here.
-    // pass 1 stages the pre-activation side output alone, pass 2 the main output without it; pass 0
-    // does the main output and writes a side output, if any, directly; pass 3 is pass 0 with an
-    // fp32 box of 32 columns (weight gradients).  Pass 8: like pass 0, and the caller has brought the
-    // aux_in block into the box with a TMA load (a thread owns a row, so loading it from global memory
-    // touches 32 lines per instruction); the result overwrites it in place.
-    if (pass == 1) {
-      uint8_t* box = stage + (c >> 1) * 16384;
-#pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        const uint32_t off = sw128_offset((uint32_t)r_in_tile, (uint32_t)((c & 1) * 4 + q));
-        *reinterpret_cast<uint4*>(box + off) =
-            make_uint4(pack_bf16x2(v[8 * q + 0], v[8 * q + 1]), pack_bf16x2(v[8 * q + 2], v[8 * q + 3]),
-                       pack_bf16x2(v[8 * q + 4], v[8 * q + 5]), pack_bf16x2(v[8 * q + 6], v[8 * q + 7]));
-      }
-      continue;
-    }
-    if ((pass == 0 || pass == 3 || pass == 8) && p.aux_out != nullptr && row_ok) {
-      uint4* dst = reinterpret_cast<uint4*>(p.aux_out + row * p.ld_aux_out + col0);
-#pragma unroll
-      for (int q = 0; q < 4; ++q)
-        dst[q] = make_uint4(pack_bf16x2(v[8 * q + 0], v[8 * q + 1]), pack_bf16x2(v[8 * q + 2], v[8 * q + 3]),
-                            pack_bf16x2(v[8 * q + 4], v[8 * q + 5]), pack_bf16x2(v[8 * q + 6], v[8 * q + 7]));
-    }
-    if (kAct != MRK_ACT_NONE && kAux != MRK_AUX_DACT) {
-#pragma unroll
-      for (int j = 0; j < 32; ++j) v[j] = apply_act<kAct>(v[j]);
-    }
-    if (kAux != MRK_AUX_NONE && (row_ok || pass == 8)) {
-      const uint4* src = reinterpret_cast<const uint4*>(p.aux_in + row * p.ld_aux_in + col0);
-#pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        const uint4 a = pass == 8 ? *reinterpret_cast<const uint4*>(stage + (c >> 1) * 16384 +
-                                                                    sw128_offset((uint32_t)r_in_tile, (uint32_t)((c & 1) * 4 + q)))
-                                  : __ldg(src + q);
-        const uint32_t w[4] = {a.x, a.y, a.z, a.w};
-#pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          const float2 f = unpack_bf16x2(w[e]);
-          if (kAux == MRK_AUX_ADD) {
-            v[8 * q + 2 * e] += f.x;
-            v[8 * q + 2 * e + 1] += f.y;
-          } else {
-            v[8 * q + 2 * e] *= apply_act_grad<kAct>(f.x);
-            v[8 * q + 2 * e + 1] *= apply_act_grad<kAct>(f.y);
-          }
-        }
-      }
-    }
-    if (pass == 3) {
-      // fp32 box: these 32 columns are one 128-byte row; the caller stores it or adds it into the output
-#pragma unroll
-      for (int q = 0; q < 8; ++q)
-        *reinterpret_cast<float4*>(stage + sw128_offset((uint32_t)r_in_tile, (uint32_t)q)) =
-            make_float4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
-      continue;
-    }
-    uint8_t* box = stage + (c >> 1) * 16384;
-#pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      const uint32_t off = sw128_offset((uint32_t)r_in_tile, (uint32_t)((c & 1) * 4 + q));
-      *reinterpret_cast<uint4*>(box + off) =
-          make_uint4(pack_bf16x2(v[8 * q + 0], v[8 * q + 1]), pack_bf16x2(v[8 * q + 2], v[8 * q + 3]),
-                     pack_bf16x2(v[8 * q + 4], v[8 * q + 5]), pack_bf16x2(v[8 * q + 6], v[8 * q + 7]));
-    }
-    continue;
   }
   if (row_ok && split_k) {
     // partial sum of one K range: reduce into the fp32 output
@@ -467,19 +393,163 @@ for (int h = 0; h < 2; ++h) {
 }
 }
 
+// Epilogue of 64 accumulator columns of one warp's 32 rows through a shared-memory box of 32 rows x 128 bytes in the
+// TMA swizzle: 64 bf16 columns, or 32 fp32 columns twice.  The warp itself hands the box to the TMA unit (`map`).
+// The box's previous store drains while the accumulator columns travel from TMEM; `free_bar` (a cluster address, or
+// 0) is told as soon as they are in registers, so that the next tile's products do not wait for the conversion.
+// Up to K = 1024 the epilogue bounds the kernel (4.4 us of products per tile at K = 1024).  With one 128-row box per
+// column half, four warps met at a barrier twice per 64 columns and then waited for the store; the parameter block,
+// passed by reference without being __grid_constant__, was read from a copy in local memory.  Measured, before ->
+// now: 8192x3072x768 45.6 -> 38.8 us, 16384x1024x1024 37.3 -> 33.2, weight gradient 3072x768x8192 43.4 -> 35.2,
+// 462x768x768 16.7 -> 13.1.
+enum StageMode {
+  kStageMain = 0,      // the output; a side output, if any, goes straight to global memory
+  kStagePreact = 1,    // the pre-activation side output alone
+  kStageNoPreact = 2,  // the output, after kStagePreact
+  kStageAuxInBox = 3,  // the output; the caller has brought the aux_in block into the box (a thread owns a row, so
+                       // loading it from global memory touches 32 lines per instruction); overwritten in place
+  kStageF32 = 4,       // fp32 output, stored
+  kStageF32Add = 5     // fp32 output, added by the TMA unit
+};
+
+template <int kAct, int kAux>
+__device__ __noinline__ void epilogue_staged_t(const GemmParams& p, uint32_t t_row, int col_base, long long row_w,
+                                               bool first_split, uint8_t* box, const CUtensorMap* map, int mode,
+                                               uint32_t free_bar) {
+  const int lane = threadIdx.x & 31;
+  const long long row = row_w + lane;
+  const bool row_ok = row < p.M;
+  const bool f32 = mode >= kStageF32;
+  const bool second = col_base + 32 < p.N;          // the second 32 columns hold anything
+  uint32_t acc[2][32];
+  tmem_ld32(t_row, acc[0]);
+  tmem_ld32(t_row + (second ? 32 : 0), acc[1]);
+  // bias: the same 64 bytes (bf16) for every lane of 32 columns
+  const bool has_bias = p.bias != nullptr && first_split;
+  const bool bias_f32 = (p.flags & MRK_GEMM_BIAS_F32) != 0;
+  const bool bias_vec = has_bias && !bias_f32 && col_base + 64 <= p.N && (reinterpret_cast<uintptr_t>(p.bias) & 15) == 0;
+  tmem_wait_ld();
+  if (free_bar != 0u) {
+    tc_fence_before();
+    __syncwarp();
+    if (lane == 0) mbar_arrive_cluster(free_bar);
+  }
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    const int col0 = col_base + h * 32;
+    float v[32];
+#pragma unroll
+    for (int j = 0; j < 32; ++j) v[j] = __uint_as_float(acc[h][j]) * p.alpha;
+    if (bias_vec) {
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        const uint4 t = __ldg(reinterpret_cast<const uint4*>(reinterpret_cast<const __nv_bfloat16*>(p.bias) + col0) + q);
+        const uint32_t w[4] = {t.x, t.y, t.z, t.w};
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const float2 f = unpack_bf16x2(w[e]);
+          v[8 * q + 2 * e] += f.x;
+          v[8 * q + 2 * e + 1] += f.y;
+        }
+      }
+    } else if (has_bias) {
+#pragma unroll
+      for (int j = 0; j < 32; ++j)
+        if (col0 + j < p.N)
+          v[j] += bias_f32 ? __ldg(reinterpret_cast<const float*>(p.bias) + col0 + j)
+                           : __bfloat162float(__ldg(reinterpret_cast<const __nv_bfloat16*>(p.bias) + col0 + j));
+    }
+    if (mode != kStagePreact) {
+      if ((mode == kStageMain || mode == kStageAuxInBox || f32) && p.aux_out != nullptr && row_ok && (h == 0 || second)) {
+        uint4* dst = reinterpret_cast<uint4*>(p.aux_out + row * p.ld_aux_out + col0);
+#pragma unroll
+        for (int q = 0; q < 4; ++q)
+          dst[q] = make_uint4(pack_bf16x2(v[8 * q + 0], v[8 * q + 1]), pack_bf16x2(v[8 * q + 2], v[8 * q + 3]),
+                              pack_bf16x2(v[8 * q + 4], v[8 * q + 5]), pack_bf16x2(v[8 * q + 6], v[8 * q + 7]));
+      }
+      if (kAct != MRK_ACT_NONE && kAux != MRK_AUX_DACT) {
+#pragma unroll
+        for (int j = 0; j < 32; ++j) v[j] = apply_act<kAct>(v[j]);
+      }
+      if (kAux != MRK_AUX_NONE && (mode == kStageAuxInBox || (row_ok && (h == 0 || second)))) {
+        const uint4* src = reinterpret_cast<const uint4*>(p.aux_in + row * p.ld_aux_in + col0);
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+          const uint4 a = mode == kStageAuxInBox
+                              ? *reinterpret_cast<const uint4*>(box + sw128_offset((uint32_t)lane, (uint32_t)(h * 4 + q)))
+                              : __ldg(src + q);
+          const uint32_t w[4] = {a.x, a.y, a.z, a.w};
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            const float2 f = unpack_bf16x2(w[e]);
+            if (kAux == MRK_AUX_ADD) {
+              v[8 * q + 2 * e] += f.x;
+              v[8 * q + 2 * e + 1] += f.y;
+            } else {
+              v[8 * q + 2 * e] *= apply_act_grad<kAct>(f.x);
+              v[8 * q + 2 * e + 1] *= apply_act_grad<kAct>(f.y);
+            }
+          }
+        }
+      }
+    }
+    if (mode != kStageAuxInBox && (h == 0 || f32)) {      // the box's last store must have read it
+      if (lane == 0) tma_store_wait_read<0>();
+      __syncwarp();
+    }
+    if (f32) {
+      if (h == 1 && !second) return;
+#pragma unroll
+      for (int q = 0; q < 8; ++q)
+        *reinterpret_cast<float4*>(box + sw128_offset((uint32_t)lane, (uint32_t)q)) =
+            make_float4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
+    } else {
+#pragma unroll
+      for (int q = 0; q < 4; ++q)
+        *reinterpret_cast<uint4*>(box + sw128_offset((uint32_t)lane, (uint32_t)(h * 4 + q))) =
+            make_uint4(pack_bf16x2(v[8 * q + 0], v[8 * q + 1]), pack_bf16x2(v[8 * q + 2], v[8 * q + 3]),
+                       pack_bf16x2(v[8 * q + 4], v[8 * q + 5]), pack_bf16x2(v[8 * q + 6], v[8 * q + 7]));
+    }
+    if (f32 || h == 1) {
+      fence_proxy_async_smem();
+      __syncwarp();
+      if (lane == 0) {
+        const int col = f32 ? col0 : col_base;
+        if (row_w < p.M) {
+          if (mode == kStageF32Add) tma_reduce_add_2d(map, smem_u32(box), col, (int32_t)row_w);
+          else tma_store_2d(map, smem_u32(box), col, (int32_t)row_w);
+        }
+        tma_store_commit();
+      }
+    }
+  }
+}
+
 // Picks the epilogue specialised for (activation, aux mode) once per tile, so the per-element code
 // has no run-time dispatch.
 __device__ __forceinline__ void epilogue_tile(const GemmParams& p, long long row, bool row_ok, uint32_t t_row,
-                                              int col_base, int ncols, bool split_k, bool first_split,
-                                              uint8_t* stage = nullptr, int r_in_tile = 0, int pass = 0) {
-#define MRK_EPI(ACT, AUX) \
-  epilogue_tile_t<ACT, AUX>(p, row, row_ok, t_row, col_base, ncols, split_k, first_split, stage, r_in_tile, pass)
+                                              int col_base, int ncols, bool split_k, bool first_split) {
+#define MRK_EPI(ACT, AUX) epilogue_tile_t<ACT, AUX>(p, row, row_ok, t_row, col_base, ncols, split_k, first_split)
 #define MRK_EPI_ACT(ACT)                                             \
   do {                                                               \
     if (p.aux_mode == MRK_AUX_ADD) MRK_EPI(ACT, MRK_AUX_ADD);        \
     else if (p.aux_mode == MRK_AUX_DACT) MRK_EPI(ACT, MRK_AUX_DACT); \
     else MRK_EPI(ACT, MRK_AUX_NONE);                                 \
   } while (0)
+  switch (p.act) {
+    case MRK_ACT_GELU_ERF: MRK_EPI_ACT(MRK_ACT_GELU_ERF); break;
+    case MRK_ACT_GELU_TANH: MRK_EPI_ACT(MRK_ACT_GELU_TANH); break;
+    case MRK_ACT_RELU: MRK_EPI_ACT(MRK_ACT_RELU); break;
+    case MRK_ACT_SILU: MRK_EPI_ACT(MRK_ACT_SILU); break;
+    default: MRK_EPI_ACT(MRK_ACT_NONE); break;
+  }
+#undef MRK_EPI
+}
+
+__device__ __forceinline__ void epilogue_staged(const GemmParams& p, uint32_t t_row, int col_base, long long row_w,
+                                                bool first_split, uint8_t* box, const CUtensorMap* map, int mode,
+                                                uint32_t free_bar) {
+#define MRK_EPI(ACT, AUX) epilogue_staged_t<ACT, AUX>(p, t_row, col_base, row_w, first_split, box, map, mode, free_bar)
   switch (p.act) {
     case MRK_ACT_GELU_ERF: MRK_EPI_ACT(MRK_ACT_GELU_ERF); break;
     case MRK_ACT_GELU_TANH: MRK_EPI_ACT(MRK_ACT_GELU_TANH); break;

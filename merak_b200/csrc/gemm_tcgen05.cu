@@ -42,7 +42,7 @@ struct SmemLayout {
 template <int BN>
 __global__ void __launch_bounds__(kNumThreads, 1)
 gemm_bf16_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ CUtensorMap tma_b,
-                 const GemmParams p) {
+                 const __grid_constant__ GemmParams p) {
   using L = SmemLayout<BN>;
   constexpr int kStages = L::kStages;
   constexpr uint32_t kTmemCols = (2 * BN <= 512) ? (2 * BN < 32 ? 32 : 2 * BN) : 512;
@@ -316,19 +316,19 @@ static int gemm_entry(const void* A, const void* B, void* C, int M, int N, int K
     p.tma_store = 0;
     if (!(flags & (MRK_GEMM_OUT_F32 | MRK_GEMM_ACCUMULATE)) && (ldc % 8) == 0 &&
         (reinterpret_cast<uintptr_t>(C) & 15) == 0) {
-      rc = make_tmap_2d(&tc, C, 2, (uint64_t)N, (uint64_t)M, (uint64_t)ldc, 64, 128, 3);
+      rc = make_tmap_2d(&tc, C, 2, (uint64_t)N, (uint64_t)M, (uint64_t)ldc, 64, 32, 3);
       if (rc) return rc;
       p.tma_store = 1;
     }
     if ((flags & MRK_GEMM_OUT_F32) && (ldc % 4) == 0 && (reinterpret_cast<uintptr_t>(C) & 15) == 0) {
-      // fp32 outputs (weight gradients): boxes of 128 rows x 32 columns, stored or added by the TMA unit
-      rc = make_tmap_2d(&tc, C, 4, (uint64_t)N, (uint64_t)M, (uint64_t)ldc, 32, 128, 3);
+      // fp32 outputs (weight gradients): boxes of 32 rows x 32 columns, stored or added by the TMA unit
+      rc = make_tmap_2d(&tc, C, 4, (uint64_t)N, (uint64_t)M, (uint64_t)ldc, 32, 32, 3);
       if (rc) return rc;
       p.tma_store = 2;
     }
     CUtensorMap taux = ta;
     if (p.tma_store && aux_out != nullptr && (ld_aux_out % 8) == 0 && (reinterpret_cast<uintptr_t>(aux_out) & 15) == 0) {
-      rc = make_tmap_2d(&taux, aux_out, 2, (uint64_t)N, (uint64_t)M, (uint64_t)ld_aux_out, 64, 128, 3);
+      rc = make_tmap_2d(&taux, aux_out, 2, (uint64_t)N, (uint64_t)M, (uint64_t)ld_aux_out, 64, 32, 3);
       if (rc) return rc;
       p.tma_store_aux = 1;
     }
@@ -336,7 +336,7 @@ static int gemm_entry(const void* A, const void* B, void* C, int M, int N, int K
     p.tma_aux_in = 0;
     if (p.tma_store == 1 && aux_mode != MRK_AUX_NONE && (ld_aux_in % 8) == 0 &&
         (reinterpret_cast<uintptr_t>(aux_in) & 15) == 0) {
-      rc = make_tmap_2d(&tauxin, aux_in, 2, (uint64_t)N, (uint64_t)M, (uint64_t)ld_aux_in, 64, 128, 3);
+      rc = make_tmap_2d(&tauxin, aux_in, 2, (uint64_t)N, (uint64_t)M, (uint64_t)ld_aux_in, 64, 32, 3);
       if (rc) return rc;
       p.tma_aux_in = 1;
     }

@@ -39,8 +39,9 @@ constexpr int kPairBBytes = (kPairBlockN / 2) * kPairBlockK * 2;  // this CTA's 
 constexpr int kPairBBoxBytes = 64 * kPairBlockK * 2;          // one 64-column box of it, in either operand layout
 constexpr int kPairSubBytes = kPairABytes + kPairBBytes;      // 32 KB per k-block
 constexpr int kPairStageBytes = kPairGroup * kPairSubBytes;   // 64 KB
-// epilogue staging: one 128-row x 64-column bf16 box (TMA-store source) per column half
-constexpr int kPairStagingBytes = 2 * 16384;
+// epilogue staging: one box of 32 rows x 128 bytes (TMA-store source) per epilogue warp
+constexpr int kPairBoxBytes = 32 * 128;
+constexpr int kPairStagingBytes = 8 * kPairBoxBytes;
 constexpr int kPairSmemTotal = kPairStages * kPairStageBytes + kPairStagingBytes + 1024 + 1024;
 
 // mode 1, store thread: the partial product of sub-tile `u` is complete in this rank's buffer.
@@ -289,7 +290,7 @@ __device__ __forceinline__ void pair_unit(const GemmParams& p, int u, int& m_blk
 __global__ void __launch_bounds__(kPairThreads, 1)
 gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ CUtensorMap tma_b,
                       const __grid_constant__ CUtensorMap tma_c, const __grid_constant__ CUtensorMap tma_aux,
-                      const __grid_constant__ CUtensorMap tma_auxin, const GemmParams p) {
+                      const __grid_constant__ CUtensorMap tma_auxin, const __grid_constant__ GemmParams p) {
   constexpr uint32_t kTmemCols = 512;   // two 256-column accumulator buffers
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
@@ -302,7 +303,7 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_co
   uint64_t* tmem_empty_bar = tmem_full_bar + 2;                     // used in the even CTA only
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tmem_empty_bar + 2);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
-  uint64_t* aux_full = reinterpret_cast<uint64_t*>(bar_base + 128);    // per column half: aux_in block has landed
+  uint64_t* aux_full = reinterpret_cast<uint64_t*>(bar_base + 128);    // per epilogue warp: aux_in block has landed
   uint64_t* pull_full = reinterpret_cast<uint64_t*>(bar_base + 256);   // mode 1, reduce phase (8 slots at most)
   uint64_t* pull_empty = pull_full + 8;
   volatile int* slot_piece = reinterpret_cast<volatile int*>(bar_base + 512);
@@ -340,8 +341,7 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_co
       mbar_init(smem_u32(&pull_full[s]), 1);
       mbar_init(smem_u32(&pull_empty[s]), 256);
     }
-    mbar_init(smem_u32(&aux_full[0]), 1);
-    mbar_init(smem_u32(&aux_full[1]), 1);
+    for (int s = 0; s < 8; ++s) mbar_init(smem_u32(&aux_full[s]), 1);
     fence_mbar_init();
     if (p.tma_aux_in) tma_prefetch_desc(&tma_auxin);
     tma_prefetch_desc(&tma_a);
@@ -468,32 +468,24 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_co
   } else {
     // ------------------------------- epilogue (both CTAs) -------------------------------
     const int quad = warp & 3;
-    const int row_in_tile = quad * 32 + lane;
     // two warps share a TMEM lane quadrant: warps 2..5 take the left half of the columns, 6..9 the right
     const int half = (warp - 2) >> 2;
-    uint8_t* stage = staging + half * 16384;        // one 128 x 64 bf16 box, reused by the two 64-column passes
-    const bool store_thread = (warp == 2 + half * 4) && lane == 0;     // issues this half's TMA stores
-    bool box_busy = false;     // a TMA store that reads the box may still be in flight
-    uint32_t aux_phase = 0;    // parity of this half's aux_in barrier
+    // Every warp stages its 32 rows in a box of its own (64 bf16 or 32 fp32 columns) and issues the TMA stores of
+    // it: no barrier joins the warps, and a store drains while its warp reads the next columns from TMEM.
+    uint8_t* box = staging + (warp - 2) * kPairBoxBytes;
+    const bool publisher = (warp == 2 + half * 4) && lane == 0;      // mode 1: reports this half's sub-tiles
+    uint64_t* aux_bar = aux_full + (warp - 2);
+    uint32_t aux_phase = 0;    // parity of this warp's aux_in barrier
     int iter = 0;
     bool ok = true;
-    int pending_flag = -1, pending_owner = 0;     // mode 1: sub-tile whose stores are in flight (store thread)
-    // before the box is overwritten: its last store must have read it (128 threads of this half)
-    auto box_acquire = [&]() __attribute__((always_inline)) {
-      if (box_busy) {
-        if (store_thread) tma_store_wait_read<0>();
-        named_bar_sync(1 + half, 128);
-      }
-    };
-    // after the box is written: one thread hands it to the TMA unit
-    auto box_store = [&](const CUtensorMap* map, int col, long long row0) __attribute__((always_inline)) {
-      fence_proxy_async_smem();
+    int pending_flag = -1, pending_owner = 0;     // mode 1: sub-tile whose stores are in flight
+    // mode 1: the stores of the previous sub-tile have landed (all four warps); tell the owner of the rows
+    auto publish_pending = [&]() __attribute__((always_inline)) {
+      if (pending_flag < 0) return;
+      if (lane == 0) tma_store_wait<0>();
       named_bar_sync(1 + half, 128);
-      if (store_thread) {
-        if (row0 < p.M) tma_store_2d(map, smem_u32(stage), col, (int32_t)row0);
-        tma_store_commit();
-      }
-      box_busy = true;
+      if (publisher) rs_publish(p, pending_owner, pending_flag);
+      pending_flag = -1;
     };
     for (int unit = cluster_id; unit < num_units && ok; unit += num_clusters, ++iter) {
       int m_blk, col0, cols;
@@ -503,8 +495,7 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_co
       const int acc = iter & 1;
       const uint32_t acc_phase = (iter >> 1) & 1;
       const long long row0 = (long long)m_blk * kPairBlockM + (long long)cta * 128;
-      const long long row = row0 + row_in_tile;
-      const bool row_ok = row < p.M;
+      const long long row_w = row0 + quad * 32;         // this warp's first row
       const uint32_t t_row = tmem_base + ((uint32_t)(quad * 32) << 16) + acc * kPairBlockN;
       const int width = cols / 2;                    // columns of each epilogue half: 128 or 64
       const int col_half = col0 + half * width;
@@ -515,100 +506,54 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_co
       // aux_in (residual, or the saved pre-activation of a backward GEMM) comes into the box by TMA
       const bool aux_tma = staged && p.tma_aux_in && p.aux_mode != MRK_AUX_NONE &&
                            !(p.tma_store_aux && p.aux_out != nullptr);
-      auto aux_fetch = [&](int col) __attribute__((always_inline)) {        // the box is free: start the load of its aux_in block
-        if (store_thread) {
-          mbar_arrive_expect_tx(smem_u32(&aux_full[half]), 16384u);
-          tma_load_2d(smem_u32(stage), &tma_auxin, smem_u32(&aux_full[half]), col, (int32_t)row0);
+      auto aux_fetch = [&](int col) __attribute__((always_inline)) {
+        if (lane == 0) {
+          tma_store_wait_read<0>();                  // the box's last store has read it
+          mbar_arrive_expect_tx(smem_u32(aux_bar), (uint32_t)kPairBoxBytes);
+          tma_load_2d(smem_u32(box), &tma_auxin, smem_u32(aux_bar), col, (int32_t)row_w);
         }
       };
-      if (aux_tma) {      // the first block's load overlaps the wait for the accumulator
-        box_acquire();
-        aux_fetch(col_half);
-      }
+      if (aux_tma) aux_fetch(col_half);              // the first block's load overlaps the wait for the accumulator
       ok = mbar_wait(smem_u32(&tmem_full_bar[acc]), acc_phase, abort_flag, p.status);
       ok = __all_sync(0xffffffffu, ok);
       if (!ok) break;
       tc_fence_after();
-      if (rs && store_thread && pending_flag >= 0) {
-        // fused reduce-scatter: the previous sub-tile's stores have landed; tell the owner of the rows
-        tma_store_wait<0>();
-        rs_publish(p, pending_owner, pending_flag);
-        pending_flag = -1;
-      }
-      auto release_tmem = [&]() __attribute__((always_inline)) {
-        tc_fence_before();
-        __syncwarp();            // every lane's TMEM reads are complete: one (possibly remote) arrival per warp
-        if (lane == 0) mbar_arrive_cluster(map_to_cta(smem_u32(&tmem_empty_bar[acc]), 0));   // TMEM is free
-      };
-      if (staged) {
-        const bool two_pass = p.tma_store_aux && p.aux_out != nullptr;
+      if (rs) publish_pending();
+      // this warp's TMEM reads of the buffer are complete: one (possibly remote) arrival per warp
+      const uint32_t free_bar = map_to_cta(smem_u32(&tmem_empty_bar[acc]), 0);
+      if (staged || staged32) {
+        const bool two_pass = staged && p.tma_store_aux && p.aux_out != nullptr;
         const int npass = (width == 128 && col_half + 64 < p.N) ? 2 : 1;        // 64-column passes with anything to write
+        const bool add = staged32 && (split_k || (p.flags & MRK_GEMM_ACCUMULATE) != 0);
         for (int b = 0; b < npass; ++b) {
           const int col_b = col_half + b * 64;
           const uint32_t t_b = t_row + half * width + b * 64;
-          if (two_pass) {
-            // the pre-activation side output of these columns first, through the same box
-            box_acquire();
-            epilogue_tile(p, row, row_ok, t_b, col_b, 64, split_k, first_split, stage, row_in_tile, 1);
-            box_store(&tma_aux, col_b, row0);
-          }
+          // the pre-activation side output of these columns first, through the same box
+          if (two_pass) epilogue_staged(p, t_b, col_b, row_w, first_split, box, &tma_aux, kStagePreact, 0u);
           if (aux_tma) {
-            if (b > 0) {
-              box_acquire();
-              aux_fetch(col_b);
-            }
-            ok = mbar_wait(smem_u32(&aux_full[half]), aux_phase, abort_flag, p.status);
+            if (b > 0) aux_fetch(col_b);
+            ok = mbar_wait(smem_u32(aux_bar), aux_phase, abort_flag, p.status);
             ok = __all_sync(0xffffffffu, ok);
             aux_phase ^= 1u;
             if (!ok) break;
-          } else {
-            box_acquire();
           }
-          epilogue_tile(p, row, row_ok, t_b, col_b, 64, split_k, first_split, stage, row_in_tile,
-                        aux_tma ? 8 : (two_pass ? 2 : 0));
-          if (b == npass - 1) release_tmem();
-          box_store(&tma_c, col_b, row0);
+          const int mode = staged32 ? (add ? kStageF32Add : kStageF32)
+                                    : (aux_tma ? kStageAuxInBox : (two_pass ? kStageNoPreact : kStageMain));
+          epilogue_staged(p, t_b, col_b, row_w, first_split, box, &tma_c, mode, b == npass - 1 ? free_bar : 0u);
         }
-        if (rs && store_thread && row0 < p.M) {
+        if (rs && row0 < p.M) {
           pending_flag = ((m_blk * p.num_n_blocks + col0 / kPairBlockN) * 2 + (int)cta) * 2 + half;
           pending_owner = (int)((row0 / p.comm.seg_rows) % p.comm.n);
         }
-      } else if (staged32) {
-        // fp32 output through the same box, 32 columns (one 128-byte row per output row) at a time: a plain
-        // store, or an element-wise add when the GEMM accumulates into its output or splits K
-        const bool add = split_k || (p.flags & MRK_GEMM_ACCUMULATE) != 0;
-        const int npass = min(width / 32, (p.N - col_half + 31) / 32);
-        for (int b = 0; b < npass; ++b) {
-          const int col_b = col_half + b * 32;
-          box_acquire();
-          epilogue_tile(p, row, row_ok, t_row + half * width + b * 32, col_b, 32, split_k, first_split,
-                        stage, row_in_tile, 3);
-          if (b == npass - 1) release_tmem();
-          fence_proxy_async_smem();
-          named_bar_sync(1 + half, 128);
-          if (store_thread) {
-            if (row0 < p.M) {
-              if (add) tma_reduce_add_2d(&tma_c, smem_u32(stage), col_b, (int32_t)row0);
-              else tma_store_2d(&tma_c, smem_u32(stage), col_b, (int32_t)row0);
-            }
-            tma_store_commit();
-          }
-          box_busy = true;
-        }
       } else {
-        epilogue_tile(p, row, row_ok, t_row + half * width, col_half, width, split_k,
-                      first_split, nullptr, row_in_tile, 0);
-        release_tmem();
+        epilogue_tile(p, row_w + lane, row_w + lane < p.M, t_row + half * width, col_half, width, split_k, first_split);
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive_cluster(free_bar);
       }
     }
-    if (store_thread) {
-      if (rs) {
-        tma_store_wait<0>();
-        if (pending_flag >= 0) rs_publish(p, pending_owner, pending_flag);
-      } else {
-        tma_store_wait_read<0>();     // shared memory stays valid until the last store has read it
-      }
-    }
+    if (rs) publish_pending();
+    else if (lane == 0) tma_store_wait_read<0>();     // shared memory stays valid until the last store has read it
     // ------------------- mode 1: reduce the sub-tiles this rank owns (all 8 epilogue warps) -------------------
     if (rs && (p.comm.phase & 2) && ok)
       rs_pull_consumer(p, smem, kPairStages * kPairStageBytes, pull_full, pull_empty, slot_piece, abort_flag);
