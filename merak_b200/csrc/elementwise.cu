@@ -648,10 +648,13 @@ act_bwd_colsum_kernel(const __nv_bfloat16* __restrict__ d, const __nv_bfloat16* 
 }
 
 // -------------------------------------------------------------------------------------------------
-// Dropout (forward, and backward with the regenerated mask), scaled casts.
+// Dropout (forward, and backward with the regenerated mask), optionally with a residual added to the result in
+// fp32 before its one rounding (a separate addition read and wrote the tensor once more: 8.7 + 6.1 us at
+// 8192 x 768), scaled casts.
 // -------------------------------------------------------------------------------------------------
 __global__ void __launch_bounds__(256)
-dropout_kernel(const __nv_bfloat16* __restrict__ x, __nv_bfloat16* __restrict__ y, long long n, float p,
+dropout_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ residual,
+               __nv_bfloat16* __restrict__ y, long long n, float p,
                const unsigned long long* __restrict__ rng, unsigned long long call_id) {
   const unsigned long long seed = rng[0], offset = rng[1];
   const float ks = 1.f / (1.f - p);
@@ -660,11 +663,15 @@ dropout_kernel(const __nv_bfloat16* __restrict__ x, __nv_bfloat16* __restrict__ 
     philox_uniform8(seed, offset + call_id, (unsigned long long)i * 8, r);
     const uint4 u = reinterpret_cast<const uint4*>(x)[i];
     const uint32_t w[4] = {u.x, u.y, u.z, u.w};
+    uint4 a = make_uint4(0u, 0u, 0u, 0u);
+    if (residual != nullptr) a = reinterpret_cast<const uint4*>(residual)[i];
+    const uint32_t aw[4] = {a.x, a.y, a.z, a.w};
     uint32_t o[4];
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
-      const float2 f = unpack_bf16x2(w[k]);
-      o[k] = pack_bf16x2(r[2 * k] < p ? 0.f : f.x * ks, r[2 * k + 1] < p ? 0.f : f.y * ks);
+      const float2 f = unpack_bf16x2(w[k]), e = unpack_bf16x2(aw[k]);
+      const float lo = r[2 * k] < p ? 0.f : f.x * ks, hi = r[2 * k + 1] < p ? 0.f : f.y * ks;
+      o[k] = residual != nullptr ? pack_bf16x2(lo + e.x, hi + e.y) : pack_bf16x2(lo, hi);
     }
     reinterpret_cast<uint4*>(y)[i] = make_uint4(o[0], o[1], o[2], o[3]);
   }
@@ -892,11 +899,17 @@ MRK_API int mrk_colsum(const void* x, float* out, long long M, int N, long long 
   return 0;
 }
 
-MRK_API int mrk_dropout(const void* x, void* y, long long n, float p, const void* rng, unsigned long long call_id, void* stream) {
+MRK_API int mrk_dropout_add(const void* x, const void* residual, void* y, long long n, float p, const void* rng,
+                            unsigned long long call_id, void* stream) {
   MRK_REQUIRE(n % 8 == 0, "dropout: element count must be a multiple of 8");
-  dropout_kernel<<<grid_for(n / 8, 256, 8), 256, 0, (cudaStream_t)stream>>>((const __nv_bfloat16*)x, (__nv_bfloat16*)y, n, p, (const unsigned long long*)rng, call_id);
+  dropout_kernel<<<grid_for(n / 8, 256, 8), 256, 0, (cudaStream_t)stream>>>(
+      (const __nv_bfloat16*)x, (const __nv_bfloat16*)residual, (__nv_bfloat16*)y, n, p, (const unsigned long long*)rng, call_id);
   MRK_CHECK_LAUNCH();
   return 0;
+}
+
+MRK_API int mrk_dropout(const void* x, void* y, long long n, float p, const void* rng, unsigned long long call_id, void* stream) {
+  return mrk_dropout_add(x, nullptr, y, n, p, rng, call_id, stream);
 }
 
 MRK_API int mrk_scaled_cast(const void* x, void* y, long long n, const float* scale_ptr, float scale, int in_f32,

@@ -41,6 +41,8 @@ int mrk_colsum(const void* x, float* out, long long M, int N, long long ld, void
 int mrk_sample_topk_topp(const void* logits, int is_bf16, long long rows, int V, long long row_stride, int top_k,
                          float top_p, float temperature, int greedy, const float* uniforms, unsigned long long seed,
                          unsigned long long step, long long* out_token, float* out_prob, void* stream);
+int mrk_dropout_add(const void* x, const void* residual, void* y, long long n, float p, const void* rng,
+                    unsigned long long call_id, void* stream);
 int mrk_dropout(const void* x, void* y, long long n, float p, const void* rng, unsigned long long call_id, void* stream);
 int mrk_scaled_cast(const void* x, void* y, long long n, const float* scale_ptr, float scale, int in_f32, int out_f32,
                     int accumulate, void* stream);

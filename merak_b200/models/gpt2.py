@@ -19,7 +19,7 @@ import torch.nn as nn
 from ..ops import gemm as G
 from ..ops.attention import flash_attention, flash_attention_packed
 from ..ops.cross_entropy import next_token_cross_entropy
-from ..ops.elementwise import dropout, embedding_sum
+from ..ops.elementwise import dropout, dropout_add
 from ..ops.linear import linear as k_linear, mlp as k_mlp
 from ..ops.modules import Dropout, Embedding, LayerNorm, Linear
 
@@ -73,18 +73,24 @@ class GPT2Attention(nn.Module):
         self.resid_pdrop = config.resid_pdrop
         self.attn_pdrop = float(config.attn_pdrop or 0.0)
 
-    def forward(self, x, residual=None):
+    def context(self, x):
+        """The heads' outputs side by side, before the output projection."""
         qkv = self.c_attn(x)
         B, L = qkv.shape[0], qkv.shape[1]     # the projection may have gathered the sequence
         local = qkv.shape[-1] // 3
         heads = local // self.head_dim
         ctx = flash_attention_packed(qkv.view(B, L, 3 * heads, self.head_dim), heads, heads, causal=True,
                                      dropout_p=self.attn_pdrop if self.training else 0.0)
-        ctx = ctx.reshape(B, L, local)
+        return ctx.reshape(B, L, local)
+
+    def forward(self, x, residual=None):
+        ctx = self.context(x)
         if residual is not None and not (self.training and self.resid_pdrop > 0):
             return self.c_proj(ctx, residual)
-        out = dropout(self.c_proj(ctx), self.resid_pdrop, self.training)
-        return out if residual is None else out + residual
+        out = self.c_proj(ctx)
+        if residual is None:
+            return dropout(out, self.resid_pdrop, self.training)
+        return dropout_add(out, residual, self.resid_pdrop, self.training)
 
 
 class GPT2MLP(nn.Module):
@@ -108,8 +114,9 @@ class GPT2MLP(nn.Module):
                 y = y + residual
         if fused_res:
             return y
-        y = dropout(y, self.resid_pdrop, self.training)
-        return y if residual is None else y + residual
+        if residual is None:
+            return dropout(y, self.resid_pdrop, self.training)
+        return dropout_add(y, residual, self.resid_pdrop, self.training)
 
 
 class GPT2Block(nn.Module):
@@ -121,8 +128,14 @@ class GPT2Block(nn.Module):
         self.mlp = GPT2MLP(config)
 
     def forward(self, hidden_states):
-        a = self.attn(self.ln_1(hidden_states), hidden_states)
-        return self.mlp(self.ln_2(a), a)
+        n, h = self.ln_1(hidden_states, return_residual=True)
+        attn = self.attn
+        if type(attn.c_proj) is Linear and self.training and attn.resid_pdrop > 0:
+            # dropout, residual and second norm are one kernel in each direction
+            n, a = self.ln_2(attn.c_proj(attn.context(n)), residual=h, p_drop=attn.resid_pdrop, return_residual=True)
+        else:
+            n, a = self.ln_2(attn(n, h), return_residual=True)
+        return self.mlp(n, a)
 
 
 class GPT2Model(nn.Module):

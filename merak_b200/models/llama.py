@@ -103,8 +103,10 @@ class LlamaDecoderLayer(nn.Module):
         self.post_attention_layernorm = RMSNorm(config.hidden_size, eps=config.rms_norm_eps)
 
     def forward(self, hidden_states, position_ids=None):
-        a = self.self_attn(self.input_layernorm(hidden_states), hidden_states, position_ids)
-        return self.mlp(self.post_attention_layernorm(a), a)
+        n, hidden_states = self.input_layernorm(hidden_states, return_residual=True)
+        a = self.self_attn(n, hidden_states, position_ids)
+        n, a = self.post_attention_layernorm(a, return_residual=True)
+        return self.mlp(n, a)
 
 
 class LlamaModel(nn.Module):

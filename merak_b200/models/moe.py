@@ -145,8 +145,9 @@ class MoEDecoderLayer(nn.Module):
         self.post_attention_layernorm = RMSNorm(c.hidden_size, eps=c.rms_norm_eps)
 
     def forward(self, hidden_states, position_ids=None):
-        a = self.self_attn(self.input_layernorm(hidden_states), hidden_states, position_ids)
-        h = self.post_attention_layernorm(a)
+        n, hidden_states = self.input_layernorm(hidden_states, return_residual=True)
+        a = self.self_attn(n, hidden_states, position_ids)
+        h, a = self.post_attention_layernorm(a, return_residual=True)
         if self.is_moe:
             return a + self.mlp(h)
         return self.mlp(h, a)

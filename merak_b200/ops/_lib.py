@@ -78,6 +78,7 @@ def _declare(lib):
     sig("mrk_act_bwd", c_int, P, P, P, P, c_ll, c_int, c_ll, c_int, P)
     sig("mrk_swiglu_bwd", c_int, P, P, P, c_ll, c_int, c_ll, P)
     sig("mrk_colsum", c_int, P, P, c_ll, c_int, c_ll, P)
+    sig("mrk_dropout_add", c_int, P, P, P, c_ll, c_float, P, c_ull, P)
     sig("mrk_dropout", c_int, P, P, c_ll, c_float, P, c_ull, P)
     sig("mrk_scaled_cast", c_int, P, P, c_ll, P, c_float, c_int, c_int, c_int, P)
     c_uint = ctypes.c_uint

@@ -264,3 +264,32 @@ def dropout(x: torch.Tensor, p: float, training: bool = True) -> torch.Tensor:
     if not _lib.use_kernels(x) or x.dtype != torch.bfloat16 or x.numel() % 8 != 0:
         return dropout_state().host_dropout(x, p)
     return _Dropout.apply(x, p)
+
+
+class _DropoutAdd(torch.autograd.Function):
+
+    @staticmethod
+    def forward(ctx, x, residual, p):
+        st = dropout_state()
+        rng = st.tensor(x.device)
+        call_id = st.next_call_id()
+        xc, rc = x.contiguous(), residual.contiguous()
+        y = torch.empty_like(xc)
+        _lib.check(_lib.kernels().mrk_dropout_add(xc.data_ptr(), rc.data_ptr(), y.data_ptr(), xc.numel(), float(p),
+                                                  rng.data_ptr(), call_id, _lib.stream_ptr()), "mrk_dropout_add")
+        ctx.rng, ctx.call_id, ctx.p = rng, call_id, p
+        return y
+
+    @staticmethod
+    def backward(ctx, dy):
+        dx = _Dropout.backward(ctx, dy)[0] if ctx.needs_input_grad[0] else None
+        return dx, dy, None
+
+
+def dropout_add(x: torch.Tensor, residual: torch.Tensor, p: float, training: bool = True) -> torch.Tensor:
+    """``dropout(x, p) + residual`` in one pass, with the mask :func:`dropout` would draw."""
+    if (p <= 0.0 or not training or not _lib.use_kernels(x, residual) or x.dtype != torch.bfloat16
+            or residual.dtype != torch.bfloat16 or x.shape != residual.shape or x.numel() % 8 != 0
+            or x.numel() == 0 or x.data_ptr() % 16 or residual.data_ptr() % 16):
+        return dropout(x, p, training) + residual
+    return _DropoutAdd.apply(x, residual, p)

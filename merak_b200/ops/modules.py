@@ -12,7 +12,7 @@ import torch.nn.functional as F
 from . import gemm as G
 from .elementwise import embedding_sum
 from .linear import linear as k_linear
-from .norm import fused_norm
+from .norm import fused_norm, norm_fork
 
 
 class Linear(nn.Linear):
@@ -24,6 +24,8 @@ class Linear(nn.Linear):
 
 class LayerNorm(nn.LayerNorm):
     def forward(self, x, residual: Optional[torch.Tensor] = None, p_drop: float = 0.0, return_residual=False):
+        if return_residual and residual is None and (p_drop == 0.0 or not self.training):
+            return norm_fork(x, self.weight, self.bias, self.eps)
         y, z = fused_norm(x, self.weight, self.bias, residual, self.eps, False, p_drop, self.training)
         return (y, z) if return_residual else y
 
@@ -36,6 +38,8 @@ class RMSNorm(nn.Module):
         self.eps = eps
 
     def forward(self, x, residual: Optional[torch.Tensor] = None, return_residual=False):
+        if return_residual and residual is None:
+            return norm_fork(x, self.weight, None, self.eps, True)
         y, z = fused_norm(x, self.weight, None, residual, self.eps, True, 0.0, self.training)
         return (y, z) if return_residual else y
 

@@ -34,7 +34,7 @@ def norm_reference(x, residual, weight, bias, eps, rms, p_drop=0.0, training=Tru
 class _FusedNorm(torch.autograd.Function):
 
     @staticmethod
-    def forward(ctx, x, residual, weight, bias, eps, rms, p_drop):
+    def forward(ctx, x, residual, weight, bias, eps, rms, p_drop, fork=False):
         H = x.shape[-1]
         x2 = x.reshape(-1, H)
         if not x2.is_contiguous():
@@ -70,6 +70,8 @@ class _FusedNorm(torch.autograd.Function):
         ctx.need_z = need_z
         if need_z:
             return y.view(x.shape), z.view(x.shape)
+        if fork:
+            return y.view(x.shape), x.view_as(x)
         return y.view(x.shape)
 
     @staticmethod
@@ -79,7 +81,9 @@ class _FusedNorm(torch.autograd.Function):
         H = shape[-1]
         if dy is None:          # only the pre-norm sum was used downstream
             if dz_extra is None:
-                return None, None, None, None, None, None, None
+                return None, None, None, None, None, None, None, None
+            if not ctx.need_z:          # fork: only the pass-through output was used
+                return dz_extra, None, None, None, None, None, None, None
             dy = torch.zeros_like(dz_extra)
         dy2 = dy.reshape(-1, H)
         if not dy2.is_contiguous():
@@ -103,7 +107,7 @@ class _FusedNorm(torch.autograd.Function):
         _lib.check(rc, "mrk_norm_bwd")
         dw = _param_grad(weight, dgamma)
         db = _param_grad(weight, dbeta) if has_bias else None
-        return dx.view(shape), (dres.view(shape) if has_res else None), dw, db, None, None, None
+        return dx.view(shape), (dres.view(shape) if has_res else None), dw, db, None, None, None, None
 
 
 def _param_grad(param, grad_f32):
@@ -143,3 +147,16 @@ def fused_norm(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tenso
         # z is x itself: keep it out of the autograd node so no output aliases an input
         return _FusedNorm.apply(x, None, weight, bias, eps, rms, 0.0), x
     return _FusedNorm.apply(x, residual, weight, bias, eps, rms, p_drop)
+
+
+def norm_fork(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tensor] = None, eps: float = 1e-5,
+              rms: bool = False) -> Tuple[torch.Tensor, torch.Tensor]:
+    """``(norm(x), x)``: a caller that feeds ``x`` both into the norm and into a residual connection takes the
+    residual from the second output.  The two gradients of ``x`` are then summed in the norm's backward kernel, in
+    fp32 and rounded once, instead of by an elementwise pass over three tensors."""
+    H = x.shape[-1]
+    if not _lib.use_kernels(x) or x.dtype != torch.bfloat16 or H % 8 != 0 or H > 8192:
+        return norm_reference(x, None, weight, bias, eps, rms, 0.0, False)[0], x
+    if not torch.is_grad_enabled():
+        return _FusedNorm.apply(x, None, weight, bias, eps, rms, 0.0), x
+    return _FusedNorm.apply(x, None, weight, bias, eps, rms, 0.0, True)
