@@ -142,8 +142,13 @@ def native():
 
 def use_kernels(*tensors) -> bool:
     """True when the inputs live on a CUDA device, i.e. the sm_100a kernels must run."""
-    return len(tensors) > 0 and all(t is None or t.is_cuda for t in tensors) and any(
-        t is not None for t in tensors)
+    found = False
+    for t in tensors:
+        if t is not None:
+            if not t.is_cuda:
+                return False
+            found = True
+    return found
 
 
 _FALLBACK_SEEN = set()
@@ -194,5 +199,8 @@ def ptr(t) -> int:
     return 0 if t is None else t.data_ptr()
 
 
-def stream_ptr() -> int:
-    return torch.cuda.current_stream().cuda_stream
+def stream_ptr(device_index: int | None = None) -> int:
+    """Raw handle of the current stream of the current device (or of ``device_index``).  Every launch asks for it:
+    ``torch.cuda.current_stream()`` builds a Stream object and probes the environment for it, 7 of the 30 us of
+    host time a launch took."""
+    return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice() if device_index is None else device_index)

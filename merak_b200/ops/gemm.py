@@ -111,14 +111,18 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn: bool = False, b_mn: bool = F
     if flop_counter.enabled():
         flop_counter.add(2 * M * N * K)
     assert a.dtype == torch.bfloat16 and b.dtype == torch.bfloat16, "tcgen05 GEMM takes bf16 operands"
-    if a.stride(1) != 1 or (a.stride(0) * 2) % 16 != 0 or a.data_ptr() % 16 != 0:
-        a = a.contiguous()
-    if b.stride(1) != 1 or (b.stride(0) * 2) % 16 != 0 or b.data_ptr() % 16 != 0:
-        b = b.contiguous()
-    if (a.stride(0) % 8) != 0 or (b.stride(0) % 8) != 0:
-        # row pitch not a multiple of 16 bytes: TMA cannot address it; pad the pitch.
-        a = _pad_pitch(a)
-        b = _pad_pitch(b)
+    (lda, sa), (ldb, sb) = a.stride(), b.stride()
+    pa, pb = a.data_ptr(), b.data_ptr()
+    if sa != 1 or sb != 1 or (lda | ldb) % 8 != 0 or (pa | pb) % 16 != 0:
+        if sa != 1 or lda % 8 != 0 or pa % 16 != 0:
+            a = a.contiguous()
+        if sb != 1 or ldb % 8 != 0 or pb % 16 != 0:
+            b = b.contiguous()
+        if a.stride(0) % 8 != 0 or b.stride(0) % 8 != 0:
+            # row pitch not a multiple of 16 bytes: TMA cannot address it; pad the pitch.
+            a = _pad_pitch(a)
+            b = _pad_pitch(b)
+        lda, ldb, pa, pb = a.stride(0), b.stride(0), a.data_ptr(), b.data_ptr()
     if out is None:
         assert not accumulate
         if N % 8 != 0:      # keep rows 16-byte aligned so the epilogue can use vector stores
@@ -150,7 +154,7 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn: bool = False, b_mn: bool = F
         assert aux_in is not None and aux_in.shape == (M, N) and aux_in.dtype == torch.bfloat16
         assert aux_in.stride(1) == 1
     rc = _lib.kernels().mrk_gemm_bf16(
-        a.data_ptr(), b.data_ptr(), out.data_ptr(), M, N, K, a.stride(0), b.stride(0), out.stride(0),
+        pa, pb, out.data_ptr(), M, N, K, lda, ldb, out.stride(0),
         _lib.ptr(bias), _lib.ptr(aux_in), aux_in.stride(0) if aux_in is not None else 0,
         _lib.ptr(pre), pre.stride(0) if pre is not None else 0, act, aux_mode, flags, float(alpha),
         block_n, _lib.stream_ptr())

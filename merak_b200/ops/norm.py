@@ -127,7 +127,7 @@ def _workspace(device, H, lib):
     """Accumulator rows for the weight / bias gradient partial sums: zero on creation, and every
     backward call leaves them zero again, so one buffer per (device, hidden size) serves all calls
     issued in stream order."""
-    key = (device.index, H, torch.cuda.current_stream(device).cuda_stream)
+    key = (device.index, H, _lib.stream_ptr(device.index))
     ws = _WORKSPACES.get(key)
     if ws is None:
         ws = _WORKSPACES[key] = torch.zeros((lib.mrk_norm_bwd_workspace_rows(), 2, H), dtype=torch.float32, device=device)
