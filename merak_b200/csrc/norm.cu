@@ -181,10 +181,16 @@ struct NormBwdParams {
   int params_f32;
 };
 
+// One block per row at a time, for hidden sizes the warp-per-row kernel does not take.  Memory bounds it, so all that a
+// row needs (its statistics and the residual gradient too) is requested one row ahead, a row costs one barrier (both
+// sums in one exchange, its buffer alternating), and no more blocks are launched than are resident: every block
+// adds 2 H floats of weight and bias gradient at its end, which at eight blocks per SM was more traffic than the
+// rows themselves.  Residual gradient included:
+// 4096 x 4096 RMS 87 -> 39 us, 3003 x 2048 RMS 30 -> 16 us, 4096 x 1600 with bias 28 -> 18 us.
 template <int THREADS, int kMaxVecPerThread>
-__global__ void __launch_bounds__(THREADS, (THREADS == 128 && kMaxVecPerThread == 1) ? 8 : 1)
+__global__ void __launch_bounds__(THREADS, kMaxVecPerThread == 4 ? 1 : (THREADS == 256 ? 2 : (kMaxVecPerThread == 2 ? 4 : 6)))
 norm_bwd_kernel(const NormBwdParams p) {
-  __shared__ float red[THREADS / 32];
+  __shared__ float2 red[2][THREADS / 32];
   const int nvec = p.H / 8;
   const bool drop = p.rng != nullptr && p.p_drop > 0.f && p.dx != nullptr;
   const float keep_scale = drop ? 1.f / (1.f - p.p_drop) : 1.f;
@@ -198,14 +204,20 @@ norm_bwd_kernel(const NormBwdParams p) {
 
   // The loads of the next row are issued before the reductions of the current one, so a block keeps
   // two rows in flight instead of stalling on DRAM between its block-wide sums.
-  uint4 raw_dy[kMaxVecPerThread], raw_z[kMaxVecPerThread];
+  uint4 raw_dy[kMaxVecPerThread], raw_z[kMaxVecPerThread], raw_e[kMaxVecPerThread];
+  float next_mean = 0.f, next_rstd = 0.f;
   auto fetch = [&](long long row) {
+    if (row < p.M) {
+      if (p.mean) next_mean = __ldg(p.mean + row);
+      next_rstd = __ldg(p.rstd + row);
+    }
 #pragma unroll
     for (int it = 0; it < kMaxVecPerThread; ++it) {
       const int vi = threadIdx.x + it * THREADS;
       if (vi < nvec && row < p.M) {
         raw_dy[it] = __ldg(reinterpret_cast<const uint4*>(p.dy + row * p.H + vi * 8));
         raw_z[it] = __ldg(reinterpret_cast<const uint4*>(p.z + row * p.H + vi * 8));
+        if (p.dz_extra) raw_e[it] = __ldg(reinterpret_cast<const uint4*>(p.dz_extra + row * p.H + vi * 8));
       }
     }
   };
@@ -215,48 +227,69 @@ norm_bwd_kernel(const NormBwdParams p) {
     for (int i = 0; i < 4; ++i) { const float2 t = unpack_bf16x2(w[i]); f[2 * i] = t.x; f[2 * i + 1] = t.y; }
   };
   fetch(blockIdx.x);
-  for (long long row = blockIdx.x; row < p.M; row += gridDim.x) {
-    const float mean = p.mean ? p.mean[row] : 0.f;
-    const float rstd = p.rstd[row];
-    float xh[kMaxVecPerThread][8], dxh[kMaxVecPerThread][8];
+  int parity = 0;
+  for (long long row = blockIdx.x; row < p.M; row += gridDim.x, parity ^= 1) {
+    const float mean = next_mean, rstd = next_rstd;
+    // the row stays packed between its two passes: unpacking twice costs less than the registers of a second block
+    uint4 cur_dy[kMaxVecPerThread], cur_z[kMaxVecPerThread], extra[kMaxVecPerThread];
     float s1 = 0.f, s2 = 0.f;
-    float dyv_all[kMaxVecPerThread][8];
 #pragma unroll
     for (int it = 0; it < kMaxVecPerThread; ++it) {
-      const int vi = threadIdx.x + it * THREADS;
-      if (vi < nvec) { unpack8(raw_dy[it], dyv_all[it]); unpack8(raw_z[it], xh[it]); }
+      cur_dy[it] = raw_dy[it];
+      cur_z[it] = raw_z[it];
+      extra[it] = raw_e[it];
     }
     fetch(row + gridDim.x);
 #pragma unroll
     for (int it = 0; it < kMaxVecPerThread; ++it) {
       const int vi = threadIdx.x + it * THREADS;
       if (vi < nvec) {
-        float g[8];
-        float (&dyv)[8] = dyv_all[it];
+        float g[8], dyv[8], xh[8];
+        unpack8(cur_dy[it], dyv);
+        unpack8(cur_z[it], xh);
         load8p(p.gamma, vi * 8, p.params_f32, g);
 #pragma unroll
         for (int i = 0; i < 8; ++i) {
-          xh[it][i] = (xh[it][i] - mean) * rstd;
-          dxh[it][i] = dyv[i] * g[i];
-          dg[it][i] += dyv[i] * xh[it][i];
+          xh[i] = (xh[i] - mean) * rstd;
+          const float dxh = dyv[i] * g[i];
+          dg[it][i] += dyv[i] * xh[i];
           db[it][i] += dyv[i];
-          s1 += dxh[it][i];
-          s2 += dxh[it][i] * xh[it][i];
+          s1 += dxh;
+          s2 += dxh * xh[i];
         }
       }
     }
-    if (p.rms) s1 = 0.f; else s1 = block_sum<THREADS>(s1, red) / p.H;
-    s2 = block_sum<THREADS>(s2, red) / p.H;
+#pragma unroll
+    for (int s = 16; s > 0; s >>= 1) {
+      s1 += __shfl_xor_sync(0xffffffffu, s1, s);
+      s2 += __shfl_xor_sync(0xffffffffu, s2, s);
+    }
+    // a warp that is a row ahead writes the other buffer; it cannot get two rows ahead
+    if ((threadIdx.x & 31) == 0) red[parity][threadIdx.x >> 5] = make_float2(s1, s2);
+    __syncthreads();
+    s1 = 0.f;
+    s2 = 0.f;
+#pragma unroll
+    for (int w = 0; w < THREADS / 32; ++w) {
+      const float2 t = red[parity][w];
+      s1 += t.x;
+      s2 += t.y;
+    }
+    s1 = p.rms ? 0.f : s1 / p.H;
+    s2 /= p.H;
 #pragma unroll
     for (int it = 0; it < kMaxVecPerThread; ++it) {
       const int vi = threadIdx.x + it * THREADS;
       if (vi < nvec) {
-        float o[8];
+        float o[8], g[8], dyv[8], xh[8];
+        unpack8(cur_dy[it], dyv);
+        unpack8(cur_z[it], xh);
+        load8p(p.gamma, vi * 8, p.params_f32, g);
 #pragma unroll
-        for (int i = 0; i < 8; ++i) o[i] = rstd * (dxh[it][i] - s1 - xh[it][i] * s2);
+        for (int i = 0; i < 8; ++i) o[i] = rstd * (dyv[i] * g[i] - s1 - (xh[i] - mean) * rstd * s2);
         if (p.dz_extra) {
           float e[8];
-          load8(p.dz_extra + row * p.H + vi * 8, e);
+          unpack8(extra[it], e);
 #pragma unroll
           for (int i = 0; i < 8; ++i) o[i] += e[i];
         }
@@ -510,14 +543,14 @@ norm_bwd_reduce_kernel(float* __restrict__ partial, int blocks, int H, float* __
 
 using namespace mrk;
 
-// Grid of the warp-per-row kernels: every block resident at once (blocks of 128 threads, no dynamic
-// shared memory), or fewer when there is less work.  The occupancy query runs once per kernel.
-template <auto kernel>
+// Grid of the row-walking kernels: every block resident at once (no dynamic shared memory), or fewer when there is
+// less work.  The occupancy query runs once per kernel.
+template <auto kernel, int THREADS = 128>
 static unsigned resident_grid(long long want) {
   static int per_sm = 0;          // one instance per kernel
   if (per_sm == 0) {
     int n = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kernel, 128, 0) != cudaSuccess || n < 1) n = 1;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kernel, THREADS, 0) != cudaSuccess || n < 1) n = 1;
     per_sm = n;
   }
   const long long cap = (long long)sm_count() * per_sm;
@@ -529,8 +562,8 @@ static void launch_norm_fwd(const NormFwdParams& p, unsigned grid, cudaStream_t 
   norm_fwd_kernel<T, V><<<grid, T, 0, s>>>(p);
 }
 template <int T, int V>
-static void launch_norm_bwd(const NormBwdParams& p, unsigned grid, cudaStream_t s) {
-  norm_bwd_kernel<T, V><<<grid, T, 0, s>>>(p);
+static void launch_norm_bwd(const NormBwdParams& p, cudaStream_t s) {
+  norm_bwd_kernel<T, V><<<resident_grid<norm_bwd_kernel<T, V>, T>(p.M), T, 0, s>>>(p);
 }
 
 MRK_API int mrk_norm_fwd(const void* x, const void* residual, const void* gamma, const void* beta, void* y,
@@ -568,8 +601,6 @@ MRK_API int mrk_norm_fwd(const void* x, const void* residual, const void* gamma,
 static void launch_norm_bwd_main(const NormBwdParams& p, cudaStream_t s) {
   const long long M = p.M;
   const int H = p.H;
-  const long long cap = (long long)sm_count() * 8;
-  const unsigned grid = (unsigned)(M < cap ? M : cap);
   if (H <= 1024 && H % 256 == 0) {
     const long long want = (M + 3) / 4;
     switch (H / 256) {
@@ -578,10 +609,10 @@ static void launch_norm_bwd_main(const NormBwdParams& p, cudaStream_t s) {
       case 3: norm_bwd_warp_kernel<3><<<resident_grid<norm_bwd_warp_kernel<3>>(want), 128, 0, s>>>(p); break;
       default: norm_bwd_warp_kernel<4><<<resident_grid<norm_bwd_warp_kernel<4>>(want), 128, 0, s>>>(p); break;
     }
-  } else if (H <= 1024) launch_norm_bwd<128, 1>(p, grid, s);
-  else if (H <= 2048) launch_norm_bwd<128, 2>(p, grid, s);
-  else if (H <= 4096) launch_norm_bwd<256, 2>(p, grid, s);
-  else launch_norm_bwd<256, 4>(p, grid, s);
+  } else if (H <= 1024) launch_norm_bwd<128, 1>(p, s);
+  else if (H <= 2048) launch_norm_bwd<128, 2>(p, s);
+  else if (H <= 4096) launch_norm_bwd<256, 2>(p, s);
+  else launch_norm_bwd<256, 4>(p, s);
 }
 
 // Number of workspace rows (each 2*H floats) mrk_norm_bwd may use.
