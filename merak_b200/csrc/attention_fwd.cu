@@ -13,11 +13,15 @@
 // accumulator traffic, and eight softmax warps per SM cannot hide several of them per block; below that lies
 // the exponential unit (1024 cycles per 128 x 128 block and SM).  So a thread reads its 128 scores ONCE into
 // registers, P goes back into the columns of S as the TMEM operand of the second product (PV_{j-1} is issued
-// before S_j, which overwrites it), and O stays in TMEM: it is rescaled only when a row maximum grows by more
-// than 2^8 over the one in use, which leaves the result the same (numerator and row sum share the factor) and
-// bf16 P its relative precision.  Measured, two 256-row tiles' warpgroups per CTA with three passes over S -> now:
-// 4096 keys causal, 32 heads of 128: 388 -> 233 us; 16 x 16 heads of 64 on 333 padded keys: 60 -> 33 us; 32 x 16
-// heads on 512 keys: 112 -> 91 us; 8 x 12 heads, 1024 keys causal, dropout: 144 -> 106 us.
+// before S_j, which overwrites it), and O stays in TMEM, where a warp rescales it once P_j is written (the scores'
+// registers are free by then: one TMEM round trip) and only if a row maximum of its 32 rows has grown.
+// P is always relative to the true running maximum, so the largest probability of a row is exactly 1 in bf16.  A
+// maximum that may lag behind by 2^8 saves most of the rescaling (82.3 instead of 84.1 us at 32 x 16 heads on 512
+// keys, 195 instead of 206 us at 4096 keys causal, 32 heads of 128), but then the largest probabilities are rounded
+// too, and peaked rows lose precision: scores of standard deviation 3 gave 0.0021 of the output's norm off fp64
+// instead of 0.0018.  Measured back to back over buffers larger than L2, two 256-row tiles' warpgroups per CTA with
+// three passes over S -> now: 4096 keys causal, 32 heads of 128: 331 -> 206 us; 16 x 16 heads of 64 on 333 padded
+// keys: 62 -> 36 us; 32 x 16 heads on 512 keys: 101 -> 84 us; 8 x 12 heads, 1024 keys causal, dropout: 148 -> 108 us.
 //
 // Replaces the eager matmul -> softmax -> dropout -> matmul attention the reference's models use
 // (examples/models/gpt2/config.py:28 forces eager attention) and the SDPA/FlashAttention-2 calls
@@ -260,24 +264,11 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__ 
       for (int i = 8; i < 128; ++i) m8[i & 7] = fmaxf(m8[i & 7], __uint_as_float(s[i >> 5][i & 31]));
       const float m_blk = fmaxf(fmaxf(fmaxf(m8[0], m8[1]), fmaxf(m8[2], m8[3])),
                                 fmaxf(fmaxf(m8[4], m8[5]), fmaxf(m8[6], m8[7]))) * sc;   // the scale is positive
-      if (j == 0) {
-        m_run = m_blk;
-      } else if (__any_sync(0xffffffffu, m_blk > m_run + 8.f)) {
-        // S_j complete means every earlier product is: nothing writes O until P_j is published
-        const float m_new = fmaxf(m_run, m_blk);
-        const float alpha = m_new == -INFINITY ? 1.f : exp2f(m_run - m_new);
-        m_run = m_new;
-        l_run *= alpha;
-#pragma unroll 1
-        for (int c = 0; c < D / 16; ++c) {
-          uint32_t o[16];
-          tmem_ld16(o_tmem + c * 16, o);
-          tmem_wait_ld();
-#pragma unroll
-          for (int i = 0; i < 16; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * alpha);
-          tmem_st16(o_tmem + c * 16, o);
-        }
-      }
+      // S_j complete means every earlier product is: nothing writes O until P_j is published
+      const bool grown = j > 0 && __any_sync(0xffffffffu, m_blk > m_run);
+      const float m_new = j > 0 ? fmaxf(m_run, m_blk) : m_blk;
+      const float alpha = m_new == -INFINITY ? 1.f : exp2f(m_run - m_new);
+      m_run = m_new;
       const float m_use = (m_run == -INFINITY) ? 0.f : m_run;
 
       // ---- probabilities -> TMEM (A operand of P V: two bf16 per column), row sum ----
@@ -303,7 +294,19 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__ 
         }
         tmem_st16(s_tmem + c * 16, packed);
       }
-      l_run += (l4[0] + l4[1]) + (l4[2] + l4[3]);
+      l_run = (grown ? l_run * alpha : l_run) + ((l4[0] + l4[1]) + (l4[2] + l4[3]));
+      if (grown) {       // the scores' registers are free: one TMEM round trip for the whole row of O
+        uint32_t o[D / 32][32];
+#pragma unroll
+        for (int c = 0; c < D / 32; ++c) tmem_ld32(o_tmem + c * 32, o[c]);
+        tmem_wait_ld();
+#pragma unroll
+        for (int c = 0; c < D / 32; ++c) {
+#pragma unroll
+          for (int i = 0; i < 32; ++i) o[c][i] = __float_as_uint(__uint_as_float(o[c][i]) * alpha);
+          tmem_st32(o_tmem + c * 32, o[c]);
+        }
+      }
       tmem_wait_st();
       tc_fence_before();
       mbar_arrive(smem_u32(p_full));

@@ -67,3 +67,37 @@ def test_rope_attention_packed(hq, hkv, D, L, given_positions):
     # dQ is summed with atomics (fp32) in both, everything else is the same arithmetic
     assert (a.grad.float() - b.grad.float()).norm() <= 2.0 ** -8 * b.grad.float().norm()
     assert torch.equal(a.grad[:, :, hq + hkv:], b.grad[:, :, hq + hkv:])
+
+
+def _blockwise(q, k, v, causal):
+    """The kernel's roundings and no others, sums in fp64: P in bf16 relative to the running row maximum over blocks of
+    128 keys, the output in bf16."""
+    q, k, v = (t.double().transpose(1, 2) for t in (q, k, v))
+    s = q @ k.transpose(-1, -2) / math.sqrt(q.shape[-1])
+    if causal:
+        s = s.masked_fill(~torch.ones(s.shape[-2:], dtype=torch.bool, device=s.device).tril(), float("-inf"))
+    m = torch.full_like(s[..., :1], float("-inf"))
+    l, o = torch.zeros_like(m), torch.zeros_like(q)
+    for j in range(0, s.shape[-1], 128):
+        new = torch.maximum(m, s[..., j:j + 128].amax(-1, keepdim=True))
+        p, alpha = torch.exp(s[..., j:j + 128] - new), torch.exp(m - new)
+        l, o = l * alpha + p.sum(-1, keepdim=True), o * alpha + p.bfloat16().double() @ v[..., j:j + 128, :]
+        m = new
+    return (o / l).transpose(1, 2).bfloat16()
+
+
+@pytest.mark.parametrize("L", [512, 1001])
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("causal", [False, True])
+@pytest.mark.parametrize("spread", [1.0, 3.0])
+def test_forward_precision(L, D, causal, spread):
+    """No further from fp64 than the roundings of P and of the output account for.  Peaked rows tell a maximum in use
+    that is not the row's own: their largest probability is then no longer exact in bf16."""
+    torch.manual_seed(L + D)
+    q = (torch.randn(2, L, 4, D, device="cuda") * spread).bfloat16()
+    k, v = (torch.randn(2, L, 4, D, device="cuda").bfloat16() for _ in range(2))
+    out = flash_attention(q, k, v, causal=causal)
+    ref = _ref(q, k, v, None, causal)
+    err, floor = (out.double() - ref).norm(), (_blockwise(q, k, v, causal).double() - ref).norm()
+    # the same roundings of nearly the same numbers; few of the 2^18 or more flip with exp2f's last bit
+    assert err <= 1.02 * floor, (err / floor).item()
