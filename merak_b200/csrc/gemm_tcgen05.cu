@@ -311,31 +311,36 @@ static int gemm_entry(const void* A, const void* B, void* C, int M, int N, int K
   MRK_REQUIRE(p.status != nullptr, "gemm: status word unavailable");
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
   if (bn == 512) {
-    // bf16 outputs that a tensor map can describe leave through shared memory + TMA stores
+    // bf16 outputs that a tensor map can describe leave through shared memory + TMA stores.  The staged epilogue reads
+    // and writes the side tensors 16 bytes at a time, bf16 ones on full-width blocks only, and with an fp32 output 32
+    // columns at a time whatever N is; what that does not fit takes the epilogue that checks every access.
+    const bool side_in = aux_mode != MRK_AUX_NONE, side_out = aux_out != nullptr;
+    const bool side_vec = (!side_in || ((ld_aux_in % 8) == 0 && (reinterpret_cast<uintptr_t>(aux_in) & 15) == 0)) &&
+                          (!side_out || ((ld_aux_out % 8) == 0 && (reinterpret_cast<uintptr_t>(aux_out) & 15) == 0));
     CUtensorMap tc = ta;
     p.tma_store = 0;
-    if (!(flags & (MRK_GEMM_OUT_F32 | MRK_GEMM_ACCUMULATE)) && (ldc % 8) == 0 &&
+    if (!(flags & (MRK_GEMM_OUT_F32 | MRK_GEMM_ACCUMULATE)) && side_vec && (ldc % 8) == 0 &&
         (reinterpret_cast<uintptr_t>(C) & 15) == 0) {
       rc = make_tmap_2d(&tc, C, 2, (uint64_t)N, (uint64_t)M, (uint64_t)ldc, 64, 32, 3);
       if (rc) return rc;
       p.tma_store = 1;
     }
-    if ((flags & MRK_GEMM_OUT_F32) && (ldc % 4) == 0 && (reinterpret_cast<uintptr_t>(C) & 15) == 0) {
+    if ((flags & MRK_GEMM_OUT_F32) && ((!side_in && !side_out) || (side_vec && N % 32 == 0)) && (ldc % 4) == 0 &&
+        (reinterpret_cast<uintptr_t>(C) & 15) == 0) {
       // fp32 outputs (weight gradients): boxes of 32 rows x 32 columns, stored or added by the TMA unit
       rc = make_tmap_2d(&tc, C, 4, (uint64_t)N, (uint64_t)M, (uint64_t)ldc, 32, 32, 3);
       if (rc) return rc;
       p.tma_store = 2;
     }
     CUtensorMap taux = ta;
-    if (p.tma_store && aux_out != nullptr && (ld_aux_out % 8) == 0 && (reinterpret_cast<uintptr_t>(aux_out) & 15) == 0) {
+    if (p.tma_store && side_out) {
       rc = make_tmap_2d(&taux, aux_out, 2, (uint64_t)N, (uint64_t)M, (uint64_t)ld_aux_out, 64, 32, 3);
       if (rc) return rc;
       p.tma_store_aux = 1;
     }
     CUtensorMap tauxin = ta;
     p.tma_aux_in = 0;
-    if (p.tma_store == 1 && aux_mode != MRK_AUX_NONE && (ld_aux_in % 8) == 0 &&
-        (reinterpret_cast<uintptr_t>(aux_in) & 15) == 0) {
+    if (p.tma_store == 1 && side_in) {
       rc = make_tmap_2d(&tauxin, aux_in, 2, (uint64_t)N, (uint64_t)M, (uint64_t)ld_aux_in, 64, 32, 3);
       if (rc) return rc;
       p.tma_aux_in = 1;
