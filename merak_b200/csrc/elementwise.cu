@@ -702,7 +702,8 @@ using namespace mrk;
 MRK_API int mrk_ce_stats(const void* logits, const long long* labels, float* stats, long long M, int V, long long ld,
                          int vocab_start, int ignore_index, int logits_f32, void* stream) {
   MRK_REQUIRE(M > 0 && V > 0, "cross entropy: empty input");
-  MRK_REQUIRE(ld % 8 == 0, "cross entropy: row pitch must be a multiple of 8 elements");
+  MRK_REQUIRE(ld % 8 == 0 && ((uintptr_t)logits & 15) == 0,
+              "cross entropy: rows must be 16-byte aligned and their pitch a multiple of 8 elements");
   cudaStream_t s = (cudaStream_t)stream;
   if (logits_f32) ce_stats_kernel<true><<<(unsigned)M, kCeThreads, 0, s>>>(logits, labels, stats, M, V, ld, vocab_start, ignore_index);
   else ce_stats_kernel<false><<<(unsigned)M, kCeThreads, 0, s>>>(logits, labels, stats, M, V, ld, vocab_start, ignore_index);
@@ -723,7 +724,8 @@ MRK_API int mrk_ce_finalize(const float* stats, int tp_parts, long long part_str
 MRK_API int mrk_ce_grad(const void* logits, const long long* labels, const float* lse, const float* grad_scale,
                         void* dlogits, long long M, int V, long long ld, long long ldd, int vocab_start,
                         int ignore_index, int logits_f32, void* stream) {
-  MRK_REQUIRE(ld % 8 == 0 && ldd % 8 == 0, "cross entropy: row pitch must be a multiple of 8 elements");
+  MRK_REQUIRE(ld % 8 == 0 && ldd % 8 == 0 && ((uintptr_t)logits & 15) == 0 && ((uintptr_t)dlogits & 15) == 0,
+              "cross entropy: rows must be 16-byte aligned and their pitch a multiple of 8 elements");
   cudaStream_t s = (cudaStream_t)stream;
   if (logits_f32) ce_grad_kernel<true><<<(unsigned)M, kCeThreads, 0, s>>>(logits, labels, lse, grad_scale, dlogits, M, V, ld, ldd, vocab_start, ignore_index);
   else ce_grad_kernel<false><<<(unsigned)M, kCeThreads, 0, s>>>(logits, labels, lse, grad_scale, dlogits, M, V, ld, ldd, vocab_start, ignore_index);

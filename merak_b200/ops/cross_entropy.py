@@ -27,7 +27,7 @@ class _SoftmaxCrossEntropy(torch.autograd.Function):
     def forward(ctx, logits, labels, ignore_index, vocab_start, tp_group, loss_scale):
         V = logits.shape[-1]
         lg = logits.reshape(-1, V)
-        if lg.stride(1) != 1 or lg.stride(0) % 8 != 0:
+        if lg.stride(1) != 1 or lg.stride(0) % 8 != 0 or lg.data_ptr() % 16 != 0:      # rows are read 16 bytes at a time
             pitch = (V + 7) // 8 * 8
             buf = torch.empty((lg.shape[0], pitch), dtype=lg.dtype, device=lg.device)
             buf[:, :V].copy_(lg)

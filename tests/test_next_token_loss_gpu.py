@@ -65,3 +65,23 @@ def test_no_row_has_a_target():
     loss = softmax_cross_entropy(logits, torch.full((3,), -100, device="cuda"))
     loss.backward()
     assert loss.item() == 0.0 and torch.count_nonzero(logits.grad) == 0
+
+
+@pytest.mark.parametrize("offset", [1, 4, 8])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+def test_logits_that_start_inside_a_row(offset, dtype):
+    """A slice of the vocabulary: rows 16-byte pitched, the first of them not 16-byte aligned (but at offset 8)."""
+    B, L, V = 3, 5, 1001
+    torch.manual_seed(offset)
+    wide = torch.randn(B, L, 1016, device="cuda").to(dtype).requires_grad_(True)
+    labels = torch.randint(0, V, (B, L), device="cuda")
+    ref_in = wide.detach().float()[..., offset:offset + V].requires_grad_(True)
+    tol = 2.0 ** -8 if dtype == torch.bfloat16 else 1e-5
+    for loss_fn, ref in ((next_token_cross_entropy, F.cross_entropy(ref_in[:, :-1].reshape(-1, V), labels[:, 1:].reshape(-1))),
+                         (softmax_cross_entropy, F.cross_entropy(ref_in.reshape(-1, V), labels.reshape(-1)))):
+        wide.grad = ref_in.grad = None
+        loss = loss_fn(wide[..., offset:offset + V], labels)
+        loss.backward()
+        ref.backward()
+        assert abs(loss.item() - ref.item()) < 1e-5 * abs(ref.item())
+        assert (wide.grad[..., offset:offset + V].float() - ref_in.grad).norm() <= tol * ref_in.grad.norm()
