@@ -99,5 +99,5 @@ def next_token_cross_entropy(logits: torch.Tensor, labels: torch.Tensor, ignore_
     if (not _lib.use_kernels(logits) or logits.dtype not in (torch.bfloat16, torch.float32) or logits.dim() != 3
             or labels.shape != logits.shape[:2] or logits.shape[1] < 2):
         return softmax_cross_entropy(logits[:, :-1, :], labels[:, 1:], ignore_index, vocab_start, tp_group)
-    shifted = F.pad(labels[:, 1:], (0, 1), value=ignore_index)
+    shifted = F.pad(labels[:, 1:].to(torch.int64), (0, 1), value=ignore_index)     # narrow types cannot hold -100
     return softmax_cross_entropy(logits, shifted, ignore_index, vocab_start, tp_group)

@@ -85,3 +85,13 @@ def test_logits_that_start_inside_a_row(offset, dtype):
         ref.backward()
         assert abs(loss.item() - ref.item()) < 1e-5 * abs(ref.item())
         assert (wide.grad[..., offset:offset + V].float() - ref_in.grad).norm() <= tol * ref_in.grad.norm()
+
+
+@pytest.mark.parametrize("dtype", [torch.bool, torch.uint8, torch.int8, torch.int32, torch.float32])
+def test_label_types(dtype):
+    """Labels of any type that the cross entropy takes, those too that cannot hold the "no target" value."""
+    torch.manual_seed(0)
+    logits = torch.randn(2, 7, 64, device="cuda", dtype=torch.bfloat16)
+    labels = torch.randint(0, 2 if dtype == torch.bool else 64, (2, 7), device="cuda").to(dtype)
+    got, want = next_token_cross_entropy(logits, labels), softmax_cross_entropy(logits[:, :-1], labels[:, 1:])
+    assert abs(got.item() - want.item()) < 1e-5 * abs(want.item())      # the same rows, summed in another order
