@@ -21,7 +21,7 @@ from ..ops.attention import flash_attention, flash_attention_packed
 from ..ops.cross_entropy import next_token_cross_entropy
 from ..ops.elementwise import dropout, dropout_add
 from ..ops.linear import linear as k_linear, mlp as k_mlp
-from ..ops.modules import Dropout, Embedding, LayerNorm, Linear
+from ..ops.modules import Dropout, Embedding, LayerNorm, Linear, norm_and_input, plain
 
 
 @dataclass
@@ -92,6 +92,8 @@ class GPT2Attention(nn.Module):
             return dropout(out, self.resid_pdrop, self.training)
         return dropout_add(out, residual, self.resid_pdrop, self.training)
 
+    own_forward = forward
+
 
 class GPT2MLP(nn.Module):
     def __init__(self, config: GPT2Config):
@@ -128,13 +130,14 @@ class GPT2Block(nn.Module):
         self.mlp = GPT2MLP(config)
 
     def forward(self, hidden_states):
-        n, h = self.ln_1(hidden_states, return_residual=True)
-        attn = self.attn
-        if type(attn.c_proj) is Linear and self.training and attn.resid_pdrop > 0:
+        n, h = norm_and_input(self.ln_1, hidden_states)
+        attn, ln_2 = self.attn, self.ln_2
+        if (attn.training and ln_2.training and attn.resid_pdrop > 0 and type(attn.c_proj) is Linear
+                and plain(attn, GPT2Attention) and plain(ln_2, LayerNorm)):
             # dropout, residual and second norm are one kernel in each direction
-            n, a = self.ln_2(attn.c_proj(attn.context(n)), residual=h, p_drop=attn.resid_pdrop, return_residual=True)
+            n, a = ln_2(attn.c_proj(attn.context(n)), residual=h, p_drop=attn.resid_pdrop, return_residual=True)
         else:
-            n, a = self.ln_2(attn(n, h), return_residual=True)
+            n, a = norm_and_input(ln_2, attn(n, h))
         return self.mlp(n, a)
 
 

@@ -19,7 +19,7 @@ import torch.nn as nn
 from ..ops.attention import rope_attention_packed
 from ..ops.cross_entropy import next_token_cross_entropy
 from ..ops.elementwise import rope_tables, swiglu
-from ..ops.modules import Embedding, Linear, RMSNorm, expose_fused_projection
+from ..ops.modules import Embedding, Linear, RMSNorm, expose_fused_projection, norm_and_input
 
 
 @dataclass
@@ -103,9 +103,9 @@ class LlamaDecoderLayer(nn.Module):
         self.post_attention_layernorm = RMSNorm(config.hidden_size, eps=config.rms_norm_eps)
 
     def forward(self, hidden_states, position_ids=None):
-        n, hidden_states = self.input_layernorm(hidden_states, return_residual=True)
+        n, hidden_states = norm_and_input(self.input_layernorm, hidden_states)
         a = self.self_attn(n, hidden_states, position_ids)
-        n, a = self.post_attention_layernorm(a, return_residual=True)
+        n, a = norm_and_input(self.post_attention_layernorm, a)
         return self.mlp(n, a)
 
 

@@ -21,7 +21,7 @@ import torch.nn.functional as F
 from ..ops.attention import flash_attention
 from ..ops.cross_entropy import next_token_cross_entropy
 from ..ops.elementwise import apply_rope, rope_tables, swiglu
-from ..ops.modules import Embedding, Linear, RMSNorm, expose_fused_projection
+from ..ops.modules import Embedding, Linear, RMSNorm, expose_fused_projection, norm_and_input
 from ..parallel.expert import MoELayer
 
 
@@ -145,9 +145,9 @@ class MoEDecoderLayer(nn.Module):
         self.post_attention_layernorm = RMSNorm(c.hidden_size, eps=c.rms_norm_eps)
 
     def forward(self, hidden_states, position_ids=None):
-        n, hidden_states = self.input_layernorm(hidden_states, return_residual=True)
+        n, hidden_states = norm_and_input(self.input_layernorm, hidden_states)
         a = self.self_attn(n, hidden_states, position_ids)
-        h, a = self.post_attention_layernorm(a, return_residual=True)
+        h, a = norm_and_input(self.post_attention_layernorm, a)
         if self.is_moe:
             return a + self.mlp(h)
         return self.mlp(h, a)

@@ -8,11 +8,23 @@ from typing import Optional
 import torch
 import torch.nn as nn
 import torch.nn.functional as F
+import torch.nn.modules.module as _torch_module
 
 from . import gemm as G
 from .elementwise import embedding_sum
 from .linear import linear as k_linear
 from .norm import fused_norm, norm_fork
+
+
+def plain(module: nn.Module, cls) -> bool:
+    """True where calling ``module`` runs the forward that ``cls`` was written with (its ``own_forward``) and nothing
+    else: no subclass, no replaced forward, no hooks.  A caller may then ask for another form of its result or run its
+    parts; whoever hooks, overrides or replaces a module sees it called, with its result as it always was."""
+    return (type(module) is cls and cls.forward is cls.own_forward and "forward" not in module.__dict__
+            and not (module._forward_hooks or module._forward_pre_hooks or module._backward_hooks
+                     or module._backward_pre_hooks or _torch_module._global_forward_hooks
+                     or _torch_module._global_forward_pre_hooks or _torch_module._global_backward_hooks
+                     or _torch_module._global_backward_pre_hooks))
 
 
 class Linear(nn.Linear):
@@ -29,6 +41,8 @@ class LayerNorm(nn.LayerNorm):
         y, z = fused_norm(x, self.weight, self.bias, residual, self.eps, False, p_drop, self.training)
         return (y, z) if return_residual else y
 
+    own_forward = forward
+
 
 class RMSNorm(nn.Module):
     def __init__(self, hidden_size: int, eps: float = 1e-6, device=None, dtype=None):
@@ -43,8 +57,18 @@ class RMSNorm(nn.Module):
         y, z = fused_norm(x, self.weight, None, residual, self.eps, True, 0.0, self.training)
         return (y, z) if return_residual else y
 
+    own_forward = forward
+
     def extra_repr(self):
         return "%d, eps=%g" % (self.weight.shape[0], self.eps)
+
+
+def norm_and_input(norm: nn.Module, x):
+    """``(norm(x), x)`` for a block that feeds ``x`` into a norm and into a residual connection; the second result
+    carries the residual (:func:`~merak_b200.ops.norm.norm_fork`)."""
+    if plain(norm, RMSNorm) or plain(norm, LayerNorm):
+        return norm(x, return_residual=True)
+    return norm(x), x
 
 
 class Embedding(nn.Embedding):
