@@ -304,6 +304,7 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_co
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tmem_empty_bar + 2);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
   uint64_t* aux_full = reinterpret_cast<uint64_t*>(bar_base + 128);    // per epilogue warp: aux_in block has landed
+  uint64_t* stored_bar = aux_full + 8;      // mode 1, per column half: a sub-tile's stores have landed (4 warps)
   uint64_t* pull_full = reinterpret_cast<uint64_t*>(bar_base + 256);   // mode 1, reduce phase (8 slots at most)
   uint64_t* pull_empty = pull_full + 8;
   volatile int* slot_piece = reinterpret_cast<volatile int*>(bar_base + 512);
@@ -342,6 +343,8 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_co
       mbar_init(smem_u32(&pull_empty[s]), 256);
     }
     for (int s = 0; s < 8; ++s) mbar_init(smem_u32(&aux_full[s]), 1);
+    mbar_init(smem_u32(&stored_bar[0]), 4);
+    mbar_init(smem_u32(&stored_bar[1]), 4);
     fence_mbar_init();
     if (p.tma_aux_in) tma_prefetch_desc(&tma_auxin);
     tma_prefetch_desc(&tma_a);
@@ -479,12 +482,19 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_co
     int iter = 0;
     bool ok = true;
     int pending_flag = -1, pending_owner = 0;     // mode 1: sub-tile whose stores are in flight
-    // mode 1: the stores of the previous sub-tile have landed (all four warps); tell the owner of the rows
+    // mode 1: the stores of the previous sub-tile have landed (all four warps); tell the owner of the rows.  The warps
+    // meet at an mbarrier: its wait is bounded and ends with the others' when a wait of another warp ran out, which a
+    // hardware barrier that this warp never reaches would not.
+    uint32_t stored_phase = 0;
     auto publish_pending = [&]() __attribute__((always_inline)) {
       if (pending_flag < 0) return;
-      if (lane == 0) tma_store_wait<0>();
-      named_bar_sync(1 + half, 128);
-      if (publisher) rs_publish(p, pending_owner, pending_flag);
+      if (lane == 0) {
+        tma_store_wait<0>();
+        mbar_arrive(smem_u32(&stored_bar[half]));
+        if (publisher && mbar_wait(smem_u32(&stored_bar[half]), stored_phase, abort_flag, p.status))
+          rs_publish(p, pending_owner, pending_flag);
+      }
+      stored_phase ^= 1u;
       pending_flag = -1;
     };
     for (int unit = cluster_id; unit < num_units && ok; unit += num_clusters, ++iter) {
