@@ -219,7 +219,8 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__ 
     const uint32_t rowkey = kDrop ? attn_drop_rowkey(attn_drop_base(p.rng[0], p.rng[1] + p.call_id),
                                                     (uint32_t)(b * p.H + h), (uint32_t)row) : 0u;
 
-    for (int j = 0; j < nb && ok; ++j) {
+    int j = 0;
+    for (; j < nb && ok; ++j) {
       const int k0 = j * kKV;
       // Key bias of this block goes to shared memory once (thread r stages key k0+r, double
       // buffered); blocks whose bias is all zero (no padding) take the unbiased path.
@@ -311,6 +312,9 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__ 
       tc_fence_before();
       mbar_arrive(smem_u32(p_full));
     }
+    // a warp whose wait ran out still meets the others at the barriers of the blocks that they go on with
+    if (!ok && kb != nullptr)
+      for (++j; j < nb; ++j) named_bar_any_nonzero(1, 0.f);
     // The output leaves through the query tile's buffer (every product that reads it is complete) as a bulk
     // tensor store: a thread holds one row, so direct stores would touch 32 lines per instruction.
     // [128 q][64] bf16 boxes in the 128-byte swizzle, D / 64 of them; rows past Lq fall outside the tensor map.
