@@ -241,7 +241,8 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__ 
       tmem_wait_ld();
 
       float sc = p.scale_log2;
-      const bool edge = (k0 + kKV > p.Lk) || (p.causal && (k0 + kKV - 1 > q0 + causal_shift));
+      // (a negative scale turns the order of the scores round: they are scaled before the maximum is taken)
+      const bool edge = (k0 + kKV > p.Lk) || (p.causal && (k0 + kKV - 1 > q0 + causal_shift)) || p.scale_log2 < 0.f;
       if (edge || has_bias) {
         const int last = p.causal ? min(p.Lk - 1, row + causal_shift) - k0 : p.Lk - 1 - k0;    // last visible column
 #pragma unroll
@@ -264,7 +265,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__ 
 #pragma unroll
       for (int i = 8; i < 128; ++i) m8[i & 7] = fmaxf(m8[i & 7], __uint_as_float(s[i >> 5][i & 31]));
       const float m_blk = fmaxf(fmaxf(fmaxf(m8[0], m8[1]), fmaxf(m8[2], m8[3])),
-                                fmaxf(fmaxf(m8[4], m8[5]), fmaxf(m8[6], m8[7]))) * sc;   // the scale is positive
+                                fmaxf(fmaxf(m8[4], m8[5]), fmaxf(m8[6], m8[7]))) * sc;   // a scale still to be applied is not negative
       // S_j complete means every earlier product is: nothing writes O until P_j is published
       const bool grown = j > 0 && __any_sync(0xffffffffu, m_blk > m_run);
       const float m_new = j > 0 ? fmaxf(m_run, m_blk) : m_blk;

@@ -101,3 +101,15 @@ def test_forward_precision(L, D, causal, spread):
     err, floor = (out.double() - ref).norm(), (_blockwise(q, k, v, causal).double() - ref).norm()
     # the same roundings of nearly the same numbers; few of the 2^18 or more flip with exp2f's last bit
     assert err <= 1.02 * floor, (err / floor).item()
+
+
+@pytest.mark.parametrize("L", [128, 300])
+@pytest.mark.parametrize("scale", [-2.0, 0.0, 2.0])
+@pytest.mark.parametrize("dropout_p", [0.0, 1e-7])
+def test_forward_scale_of_any_sign(L, scale, dropout_p):
+    """Scores some hundreds wide: probabilities relative to anything but the row's maximum overflow."""
+    torch.manual_seed(L)
+    q, k, v = (torch.randn(1, L, 2, 64, device="cuda").bfloat16() for _ in range(3))
+    out = flash_attention(4 * q, 4 * k, v, scale=scale, dropout_p=dropout_p)     # at 1e-7 no probability is dropped
+    ref = _ref(4 * q * (scale * 8.0), 4 * k, v, None, False)                     # (the oracle divides by 8)
+    assert (out.double() - ref).norm() <= 2.0 ** -7 * ref.norm()
