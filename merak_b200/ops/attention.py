@@ -216,7 +216,7 @@ class _RopeAttentionPacked(torch.autograd.Function):
     @staticmethod
     def forward(ctx, qkv, hq, hkv, cos, sin, positions, causal, scale):
         if not _tma_ok(qkv):
-            qkv = qkv.contiguous()
+            qkv = qkv.clone(memory_format=torch.contiguous_format)     # contiguous at an odd address needs a copy too
         B, L, _, D = qkv.shape
         qk = _rope_launch(qkv[:, :, :hq + hkv], cos, sin, positions, False)
         q, k, v = qk[:, :, :hq], qk[:, :, hq:], qkv[:, :, hq + hkv:]

@@ -113,3 +113,15 @@ def test_forward_scale_of_any_sign(L, scale, dropout_p):
     out = flash_attention(4 * q, 4 * k, v, scale=scale, dropout_p=dropout_p)     # at 1e-7 no probability is dropped
     ref = _ref(4 * q * (scale * 8.0), 4 * k, v, None, False)                     # (the oracle divides by 8)
     assert (out.double() - ref).norm() <= 2.0 ** -7 * ref.norm()
+
+
+def test_rope_attention_packed_at_an_odd_address():
+    cos, sin = rope_tables(64, 64, device="cuda")
+    base = torch.randn(1 + 2 * 37 * 12 * 64, device="cuda").bfloat16()
+    odd = base[1:].view(2, 37, 12, 64).requires_grad_(True)
+    even = odd.detach().clone().requires_grad_(True)
+    g = torch.randn(2, 37, 4, 64, device="cuda").bfloat16()
+    outs = [rope_attention_packed(t, 4, 4, cos, sin) for t in (odd, even)]
+    for o in outs:
+        o.backward(g)
+    assert torch.equal(*outs) and (odd.grad.float() - even.grad.float()).norm() <= 2.0 ** -8 * even.grad.float().norm()
