@@ -399,9 +399,9 @@ for (int h = 0; h < 2; ++h) {
 // 0) is told as soon as they are in registers, so that the next tile's products do not wait for the conversion.
 // Up to K = 1024 the epilogue bounds the kernel (4.4 us of products per tile at K = 1024).  With one 128-row box per
 // column half, four warps met at a barrier twice per 64 columns and then waited for the store; the parameter block,
-// passed by reference without being __grid_constant__, was read from a copy in local memory.  Measured, before ->
-// now: 8192x3072x768 45.6 -> 38.8 us, 16384x1024x1024 37.3 -> 33.2, weight gradient 3072x768x8192 43.4 -> 35.2,
-// 462x768x768 16.7 -> 13.1.
+// passed by reference without being __grid_constant__, was read from a copy in local memory.  Medians of 24 alternating
+// samples of 8 launches over buffers larger than L2, before -> now: 8192x3072x768 48.3 -> 42.6 us, 16384x1024x1024
+// 40.1 -> 36.2, weight gradient 3072x768x8192 45.2 -> 38.0, 462x768x768 17.0 -> 13.2.
 enum StageMode {
   kStageMain = 0,      // the output; a side output, if any, goes straight to global memory
   kStagePreact = 1,    // the pre-activation side output alone

@@ -29,10 +29,12 @@ constexpr int kPairThreads = 320;     // TMA warp, UMMA warp, 8 epilogue warps
 constexpr int kPairGroup = 2;
 constexpr int kPairStages = 3;
 // Time of a 256-column and of a 128-column unit, relative: half the products, but A is loaded in full (24 instead of
-// 32 KB per k-block for half the math) and the fill and the drain of a unit stay.  Measured on B200, whole tiles
-// only -> with halves where the rule takes them: 8192x3072x768 87 -> 75 us, 16384x1024x1024 45 -> 42, 8192x50257x768
-// 605 -> 560, 3003x2048x2048 48 -> 44; at a cost of 50 the rule also halves tiles of long products that lose by it
-// (4096x4096x11008 259 -> 286 us), at 75 it leaves 8192x3072x768 whole.
+// 32 KB per k-block for half the math) and the fill and the drain of a unit stay.  Only that a half takes at least
+// half as long as a whole and less than a whole matters: any such pair of costs picks the same split.  Medians of 24
+// alternating samples of 8 launches over buffers larger than L2, whole tiles only -> halves where the rule takes them:
+// 462x3072x768 17.2 -> 15.1 us, 4000x4096x1024 37.6 -> 35.5, 8192x3072x768 55.8 -> 53.9, 16384x1024x1024 48.0 -> 45.5,
+// 4096x4096x4096 105.9 -> 103.4.  The gain is a fraction of one unit, so it fades with the rounds (8192x50257x768 594.7
+// -> 596.7) and with K (4096x4096x11008 260.4 -> 260.6), both inside their spread; none of 48 shapes lost by it.
 constexpr int kPairFullCost = 100, kPairHalfCost = 60;
 constexpr int kPairABytes = 128 * kPairBlockK * 2;            // this CTA's rows of A, one k-block
 constexpr int kPairBBytes = (kPairBlockN / 2) * kPairBlockK * 2;  // this CTA's half of B, one k-block
@@ -589,13 +591,9 @@ static int pair_full_tiles(int tiles, int strip, int clusters) {
   long long best_cost = 0;
   for (int o = 0; o < 4; ++o) {
     const int full = options[o], halves = 2 * (tiles - full) + strip;
-    long long cost = 0;                               // of the cluster with most to do; units go round robin
-    for (int c = 0; c < clusters; ++c) {
-      const long long nf = c < full ? (full - 1 - c) / clusters + 1 : 0;
-      const long long all = c < full + halves ? (full + halves - 1 - c) / clusters + 1 : 0;
-      const long long t = nf * kPairFullCost + (all - nf) * kPairHalfCost;
-      if (t > cost) cost = t;
-    }
+    // units go round robin, whole tiles first: the first cluster has the most of both
+    const long long cost = (long long)((full + halves + clusters - 1) / clusters) * kPairHalfCost +
+                           (long long)((full + clusters - 1) / clusters) * (kPairFullCost - kPairHalfCost);
     if (o == 0 || cost < best_cost) { best_cost = cost; best = full; }
   }
   return best;
