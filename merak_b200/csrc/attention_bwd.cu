@@ -41,11 +41,6 @@ constexpr int kBwdThreads = 320;
 struct AttnBwdParams {
   const float* lse;        // [B, H, Lq]
   const float* delta;      // [B, H, Lq]  rowsum(dO o O)
-  float* dq_acc;           // [B, Lq, H, D] fp32, zero-initialised
-  __nv_bfloat16* dk;       // [B, Lk, Hkv, D] strides below
-  __nv_bfloat16* dv;
-  long long dk_sb, dk_ss, dk_sh;
-  long long dv_sb, dv_ss, dv_sh;
   const float* key_bias;   // optional [B, Lk]
   int B, H, Hkv, Lq, Lk;
   int causal;
@@ -691,10 +686,7 @@ MRK_API int mrk_attn_bwd_drop(const void* q, const void* k, const void* v, const
     MRK_CHECK_LAUNCH();
   }
   AttnBwdParams p;
-  p.lse = lse; p.delta = delta; p.dq_acc = dq_acc;
-  p.dk = (__nv_bfloat16*)dk; p.dv = (__nv_bfloat16*)dv;
-  p.dk_sb = sdk[0]; p.dk_ss = sdk[1]; p.dk_sh = sdk[2];
-  p.dv_sb = sdv[0]; p.dv_ss = sdv[1]; p.dv_sh = sdv[2];
+  p.lse = lse; p.delta = delta;
   p.key_bias = key_bias;
   p.B = B; p.H = H; p.Hkv = Hkv; p.Lq = Lq; p.Lk = Lk; p.causal = causal;
   p.scale = scale; p.scale_log2 = scale * 1.4426950408889634f;

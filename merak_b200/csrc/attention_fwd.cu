@@ -36,8 +36,6 @@ namespace mrk {
 constexpr int kKV = 128;  // keys per block
 
 struct AttnFwdParams {
-  __nv_bfloat16* out;           // [B, Lq, H, D] with strides below
-  long long o_sb, o_ss, o_sh;   // batch / seq / head strides (elements)
   float* lse;                   // [B, H, Lq]
   const float* key_bias;        // optional [B, Lk], added to every score column
   int B, H, Hkv, Lq, Lk;
@@ -416,8 +414,6 @@ MRK_API int mrk_attn_fwd_drop(const void* q, const void* k, const void* v, void*
   CUtensorMap to;
   if ((rc = make_bshd_tmap(&to, out, D, Lq, H, B, o_sb, o_ss, o_sh, 128))) return rc;
   AttnFwdParams p;
-  p.out = reinterpret_cast<__nv_bfloat16*>(out);
-  p.o_sb = o_sb; p.o_ss = o_ss; p.o_sh = o_sh;
   p.lse = lse; p.key_bias = key_bias;
   p.B = B; p.H = H; p.Hkv = Hkv; p.Lq = Lq; p.Lk = Lk;
   p.causal = causal;

@@ -3,8 +3,9 @@
 Forward makes one pass over the logits producing per-row ``(max, sum-exp, target logit)``; with a
 tensor-parallel group the triples of all ranks are exchanged in ONE all-gather (the reference
 issues three all-reduces: Merak/core/mpu/cross_entropy.py:33,64,72) and merged on device.  The
-gradient ``(softmax - onehot) * scale`` is written by a second kernel that reads the still
-L2-resident rows.  Mean reduction over non-ignored targets, like ``nn.CrossEntropyLoss``.
+gradient ``(softmax - onehot) * scale`` is written by a second kernel that reads the rows again.
+Mean reduction over non-ignored targets, like ``nn.CrossEntropyLoss``; rows without a target are
+not read, their gradient is zero whatever they hold (``nn.CrossEntropyLoss`` hands a NaN on there).
 """
 from __future__ import annotations
 
