@@ -73,7 +73,7 @@ __device__ __forceinline__ bool named_bar_any_nonzero(uint32_t bar_id, float v) 
 }
 
 // kDrop: dropout on the probabilities.  A template argument, because a branch in the element loop cuts it into
-// pieces of four exponentials whose latency nothing hides (96 -> 91 us at 32 x 16 heads on 512 keys).
+// pieces of four exponentials whose latency nothing hides (5 % of the kernel without dropout, at 512 keys).
 template <int D, bool kDrop>
 __global__ void __launch_bounds__(AttnFwdSmem<D>::kThreads, 2)
 attn_fwd_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__ CUtensorMap tk,

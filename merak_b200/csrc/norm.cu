@@ -79,8 +79,9 @@ __device__ __forceinline__ float block_sum_once(float v, float (&red)[THREADS / 
 }
 
 // One block per row at a time, for hidden sizes the warp-per-row kernel does not take: as many blocks as are resident,
-// the next row's loads issued before this row's sums, one barrier per sum.  4096 x 4096 RMS
-// 27 -> 19 us, 4096 x 1600 with bias 13.0 -> 10.7 us, 3003 x 2048 RMS 7.8 -> 6.9 us.
+// the next row's loads issued before this row's sums, one barrier per sum.  Medians of 24 alternating samples of 8
+// launches over buffers larger than L2, a block per row with four barriers -> now: 4096 x 4096 RMS 24.9 -> 16.8 us, 4096 x
+// 1600 with bias 14.7 -> 12.5 us, 3003 x 2048 RMS 10.5 -> 8.6 us.
 template <int THREADS, int kMaxVecPerThread>
 __global__ void __launch_bounds__(THREADS, kMaxVecPerThread == 4 ? 2 : (THREADS == 256 ? 4 : 8))
 norm_fwd_kernel(const NormFwdParams p) {
@@ -205,8 +206,8 @@ struct NormBwdParams {
 // row needs (its statistics and the residual gradient too) is requested one row ahead, a row costs one barrier (both
 // sums in one exchange, its buffer alternating), and no more blocks are launched than are resident: every block
 // adds 2 H floats of weight and bias gradient at its end, which at eight blocks per SM was more traffic than the
-// rows themselves.  Residual gradient included:
-// 4096 x 4096 RMS 87 -> 39 us, 3003 x 2048 RMS 30 -> 16 us, 4096 x 1600 with bias 28 -> 18 us.
+// rows themselves.  Residual gradient and the reduction over the blocks included, measured as the forward kernel was:
+// 4096 x 4096 RMS 87 -> 42 us, 3003 x 2048 RMS 38 -> 23 us, 4096 x 1600 with bias 47 -> 24 us.
 template <int THREADS, int kMaxVecPerThread>
 __global__ void __launch_bounds__(THREADS, kMaxVecPerThread == 4 ? 1 : (THREADS == 256 ? 2 : (kMaxVecPerThread == 2 ? 4 : 6)))
 norm_bwd_kernel(const NormBwdParams p) {
