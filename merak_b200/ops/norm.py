@@ -142,6 +142,9 @@ def fused_norm(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tenso
         p_drop = 0.0
     H = x.shape[-1]
     if not _lib.use_kernels(x) or x.dtype != torch.bfloat16 or H % 8 != 0 or H > 8192:
+        if p_drop > 0.0:          # the dropout kernel takes more widths; a host mask would be baked into a captured step
+            from .elementwise import dropout
+            x, p_drop = dropout(x, p_drop), 0.0
         return norm_reference(x, residual, weight, bias, eps, rms, p_drop, training)
     if residual is None and p_drop == 0.0:
         # z is x itself: keep it out of the autograd node so no output aliases an input

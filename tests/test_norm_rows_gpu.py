@@ -72,3 +72,30 @@ def test_every_row(H, rms, form):
     for got, want in ((w, wd), (b, bd)):
         if got is not None:
             assert (got.grad.double() - want.grad).norm() <= 2.0 ** -8 * want.grad.norm()
+
+
+@pytest.mark.parametrize("H", [100, 8200])
+def test_dropout_of_widths_the_norm_kernel_does_not_take(H):
+    """The mask is the dropout kernel's, drawn on the device: a captured call draws a new one at every replay."""
+    st = dropout_state()
+    x, r = torch.randn(16, H, device="cuda").bfloat16(), torch.randn(16, H, device="cuda").bfloat16()
+    w, b = torch.randn(H, device="cuda").bfloat16(), torch.randn(H, device="cuda").bfloat16()
+
+    def want():
+        st.set_call_id(3)
+        return (dropout(x, 0.25).float() + r.float()).bfloat16()
+
+    st.set_call_id(3)
+    y, z = fused_norm(x, w, b, r, EPS, False, 0.25)
+    assert torch.equal(z, want())
+    assert torch.allclose(y.float(), _norm(z.float(), w.float(), b.float(), False), atol=0.05, rtol=2.0 ** -7)
+    graph = torch.cuda.CUDAGraph()
+    st.set_call_id(3)
+    with torch.cuda.graph(graph):
+        captured = fused_norm(x, w, b, r, EPS, False, 0.25)[1]
+    for _ in range(2):
+        graph.replay()
+        assert torch.equal(captured, want())
+        st.advance_micro()
+    graph.replay()
+    assert torch.equal(captured, want()) and not torch.equal(captured, z)
