@@ -95,3 +95,13 @@ def test_label_types(dtype):
     labels = torch.randint(0, 2 if dtype == torch.bool else 64, (2, 7), device="cuda").to(dtype)
     got, want = next_token_cross_entropy(logits, labels), softmax_cross_entropy(logits[:, :-1], labels[:, 1:])
     assert abs(got.item() - want.item()) < 1e-5 * abs(want.item())      # the same rows, summed in another order
+
+
+def test_labels_of_another_shape_take_the_sliced_path():
+    torch.manual_seed(0)
+    logits = torch.randn(2, 4, 16, device="cuda").bfloat16().requires_grad_(True)
+    labels = torch.randint(0, 16, (2, 4, 1), device="cuda")
+    loss = next_token_cross_entropy(logits, labels)
+    loss.backward()
+    want = F.cross_entropy(logits[:, :-1].float().reshape(-1, 16), labels[:, 1:].reshape(-1))
+    assert abs(loss.item() - want.item()) < 1e-5 and torch.count_nonzero(logits.grad[:, -1]) == 0
